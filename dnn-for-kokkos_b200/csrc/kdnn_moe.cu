@@ -907,7 +907,9 @@ __global__ void __launch_bounds__(kGateThreads) moe_gate_kernel(const GateParams
   float* rwts = reinterpret_cast<float*>(ridx + RT * p.top_k);                          // [RT][top_k]
   float* part = rwts + RT * p.top_k;                                     // [16 warps][TPC][32] partial logits
   // bf16 tokens: a second copy of the rows as stored, [8][H + 32] (rows past nt are zero), for the tensor-core product
-  __nv_bfloat16* xb = reinterpret_cast<__nv_bfloat16*>(part + (kGateThreads / 32) * TPC * 32);
+  // (read and written 16 bytes at a time; the float arrays in front of it end on any 4-byte boundary)
+  const size_t xb_off = (reinterpret_cast<uint8_t*>(part + (kGateThreads / 32) * TPC * 32) - gate_smem + 15) & ~size_t(15);
+  __nv_bfloat16* xb = reinterpret_cast<__nv_bfloat16*>(gate_smem + xb_off);
   constexpr bool kTensor = std::is_same<ST, __nv_bfloat16>::value;
   const int xb_pitch = p.H + 32;
   __shared__ int s_last;
@@ -951,8 +953,10 @@ __global__ void __launch_bounds__(kGateThreads) moe_gate_kernel(const GateParams
     const ST* rw = static_cast<const ST*>(p.rw);
     constexpr int kWarps = kGateThreads / 32;
     const int Ec = (p.E + C - 1) / C, e_lo = static_cast<int>(crank) * Ec, e_hi = min(p.E, e_lo + Ec);
-    const int kw = p.H / kWarps, k_lo = warp * kw;          // this warp's piece of K (a multiple of 16 elements)
     if (kTensor) {
+      // this warp's piece of K: whole 32-element steps (an even split when H is a multiple of 512)
+      const int k_lo = static_cast<int>(static_cast<unsigned>(warp * (p.H / 32)) / kWarps) * 32;
+      const int kw = static_cast<int>(static_cast<unsigned>((warp + 1) * (p.H / 32)) / kWarps) * 32 - k_lo;
       // bf16: the product runs on the tensor cores (mma.sync m16n8k16, fp32 accumulators): experts are the M
       // rows, the (up to eight) tokens the N columns. A lane takes 16 bytes of an expert row and of a token row
       // at the same place, which is the fragment of TWO k-steps under one fixed permutation of the 32 elements
@@ -1012,6 +1016,7 @@ __global__ void __launch_bounds__(kGateThreads) moe_gate_kernel(const GateParams
       }
     } else
     for (int eb = e_lo; eb < e_hi; eb += 32) {
+      const int kw = p.H / kWarps, k_lo = warp * kw;        // this warp's piece of K (a multiple of 16 elements)
       const int e = eb + lane;
       const bool live = e < e_hi;
       const ST* row = rw + static_cast<size_t>(live ? e : eb) * p.ldr + k_lo;
@@ -1479,7 +1484,7 @@ cudaError_t moe_block_launch(const BlockArgs& a, cudaStream_t st) {
   auto gate_smem = [&](int n) {
     const size_t rt = (n + kGateCluster - 1) / kGateCluster;
     return std::max(((size_t)n * H + rt * (2 * E + 2 * S) + (size_t)(kGateThreads / 32) * n * 32) * sizeof(float),
-                    (a.e_count + 1) * sizeof(int)) + (a.scalar == KDNN_BF16 ? 8 * (H + 32) * 2 : 0);
+                    (a.e_count + 1) * sizeof(int)) + (a.scalar == KDNN_BF16 ? 16 + 8 * (H + 32) * 2 : 0);
   };
   while (tpc > 1 && gate_smem(tpc) > 200 * 1024) tpc >>= 1;
   const size_t gsm = gate_smem(tpc);

@@ -83,6 +83,13 @@ def test_moe_block_small(kd, port, dtype, kind):
     _block_case(kd, port, 8, 2, 512, 512, 13, dtype, 11, kind, ref=ref)
 
 
+@pytest.mark.parametrize("E,k,H,T", [(8, 1, 512, 5), (9, 2, 768, 3), (6, 2, 1280, 70)])
+def test_moe_block_odd_expert_counts_and_uneven_k_pieces(kd, port, E, k, H, T):
+    """E + top_k odd moves the shared-memory arrays of the gate kernel off 16 bytes; H that is not a multiple of
+    512 gives its warps uneven pieces of the router product."""
+    _block_case(kd, port, E, k, H, 256, T, torch.bfloat16, 21)
+
+
 def test_moe_block_sigmoid_router_with_bias(kd, port):
     _block_case(kd, port, 16, 4, 512, 256, 9, torch.float32, 12, sigmoid=True, bias=True)
 
