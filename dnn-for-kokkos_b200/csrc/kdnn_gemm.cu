@@ -3,6 +3,7 @@
 // holds all M activation rows. Row m of Y equals the decode GEMV applied to row m.
 #include "kdnn_grouped.cuh"
 #include "kdnn_mma.cuh"
+#include "kdnn_split.cuh"
 #include "kdnn_tc.cuh"
 
 namespace kdnn {
@@ -18,7 +19,7 @@ static size_t gemm_items_offset(size_t M) {
   return gemm_groups_offset(M) + (((M + kTcNT - 1) / kTcNT * sizeof(int4) + 255) & ~size_t(255));
 }
 size_t gemm_workspace_bytes(size_t M, size_t K) {
-  const size_t a = M * (K / 64) * sizeof(ActItem), b = M * act_row_pitch(K);
+  const size_t a = M * (K / 64) * sizeof(ActItem), b = M * act_row_pitch_max(K);
   return gemm_items_offset(M) + (a > b ? a : b);
 }
 
@@ -47,6 +48,38 @@ static int gemm_tile_rows(size_t N, size_t groups) {
   return 128;
 }
 
+// Q4_K rows against M activation rows on the split-fp16 tensor-core kernel: the row quantizer and one tile launch.
+static cudaError_t gemm_split(const void* w, size_t N, size_t K, const void* X, size_t ldx, size_t M, int xs, void* Y,
+                              size_t ldy, int ys, uint8_t* b, cudaStream_t st) {
+  int* n_groups = reinterpret_cast<int*>(b) + 2;
+  int4* groups  = reinterpret_cast<int4*>(b + gemm_groups_offset(M));
+  uint8_t* xrows = b + gemm_items_offset(M);
+  SplitParams q{};
+  cudaError_t err = moe_status_ptr(&q.status);
+  if (err != cudaSuccess) return err;
+  // Two row tiles per activation stage and 64-row groups once that fills the chip; below, one row tile per CTA, its
+  // rows chosen so that every SM gets the same number of tiles, and 32-row groups.
+  const size_t sms = static_cast<size_t>(device_sm_count());
+  const bool wide = M > 32 && (N + 255) / 256 * ((M + 63) / 64) >= sms;
+  const int cap = wide ? 64 : 32;
+  const size_t ngroups = (M + cap - 1) / cap;
+  q.tile_rows = wide ? 128 : gemm_tile_rows(N, ngroups);
+  q.box_rows = q.tile_rows; q.boxes = 1;
+  const size_t unit_rows = static_cast<size_t>(q.tile_rows) * (wide ? 2 : 1);
+  q.row_units = (int)((N + unit_rows - 1) / unit_rows);
+  err = tc_encode_matrix(&q.one, w, N, row_bytes_of(KDNN_GGML_Q4_K, K), q.box_rows);
+  if (err != cudaSuccess) return err;
+  err = xs == KDNN_F32
+            ? launch_split_rows<float>(static_cast<const float*>(X), ldx, (int)M, (int)K, xrows, groups, n_groups, cap, st)
+            : launch_split_rows<__nv_bfloat16>(static_cast<const __nv_bfloat16*>(X), ldx, (int)M, (int)K, xrows, groups, n_groups, cap, st);
+  if (err != cudaSuccess) return err;
+  q.N = (int)N; q.K = (int)K; q.groups = groups; q.n_groups = n_groups; q.S = 1;
+  q.xrows = xrows; q.x_pitch = split_row_pitch(K, 256); q.dst = Y; q.ld_dst = ldy;
+  const int units = (int)(ngroups * q.row_units);
+  if (wide) return ys == KDNN_F32 ? launch_grouped_split<2, 2, 2, 1, float>(q, units, st) : launch_grouped_split<2, 2, 2, 1, __nv_bfloat16>(q, units, st);
+  return ys == KDNN_F32 ? launch_grouped_split<2, 1, 1, 1, float>(q, units, st) : launch_grouped_split<2, 1, 1, 1, __nv_bfloat16>(q, units, st);
+}
+
 // `dots` (parity probe, tcgen05 kernel only): int32 [M][N][K/32] raw sub-block dots, or nullptr.
 cudaError_t gemm_launch(uint32_t dt, const void* w, size_t N, size_t K, const void* X, size_t ldx,
                         size_t M, int xs, void* Y, size_t ldy, int ys, void* ws, int32_t* dots, cudaStream_t st) {
@@ -67,7 +100,9 @@ cudaError_t gemm_launch(uint32_t dt, const void* w, size_t N, size_t K, const vo
       }
       return cudaSuccess;
     }
-    kind = M <= 8 ? 2 : 1;
+    if (dt == KDNN_GGML_Q4_K && (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && tc_encode_fn() != nullptr)
+      return gemm_split(w, N, K, X, ldx, M, xs, Y, ldy, ys, b, st);
+    kind = 1;
   } else if (kind == 3) {
     kind = 2;
   }

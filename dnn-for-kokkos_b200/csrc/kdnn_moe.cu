@@ -15,6 +15,7 @@
 #include <type_traits>
 #include "kdnn_grouped.cuh"
 #include "kdnn_mma.cuh"
+#include "kdnn_split.cuh"
 #include "kdnn_tc.cuh"
 
 #include <limits.h>
@@ -366,13 +367,14 @@ __global__ void moe_sort_kernel(const int32_t* idx, int n_slots, int e_first,
 // its expert's run is a prefix popcount -- every slot is placed independently, in token order, by its own
 // thread (no sweep per expert). A token that names the same expert twice (callers may pass any idx) is
 // detected by the atomicOr that sets the bit; the kernel then places sequentially per expert instead.
-//   groups[g] = {table index of the expert, first position, rows (<= 32), 0}: one entry per 32 rows of an
+//   groups[g] = {table index of the expert, first position, rows (<= cap), 0}: one entry per cap = 2^cap_log2 rows of an
 //   expert's run, experts without rows have none.
 struct PrepParams {
   const int32_t* idx;
   int n_slots, S, e_first, e_count, words;   // words = ceil(T / 32)
   int* offs; int* list; int* pos; int4* groups; int* n_groups;
   const void* X; size_t ldx; int T, H; uint8_t* xrows; size_t x_pitch;   // X == nullptr: no rows to quantize
+  int cap_log2;                              // activation rows per group: 32 or 64
 };
 
 __device__ void moe_sort_block(const PrepParams& p, uint32_t* sm) {
@@ -425,7 +427,7 @@ __device__ void moe_sort_block(const PrepParams& p, uint32_t* sm) {
     for (int e0 = 0; e0 < E; e0 += 32) {
       const int e = e0 + tid;
       const int c = e < E ? counts[e] : 0;
-      const int gc = (c + kTcNT - 1) / kTcNT;
+      const int gc = (c + (1 << p.cap_log2) - 1) >> p.cap_log2;
       int incl = c, gincl = gc;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -446,8 +448,8 @@ __device__ void moe_sort_block(const PrepParams& p, uint32_t* sm) {
   for (int e = tid; e < E; e += nt) {
     p.offs[e] = starts[e];
     const int c = counts[e];
-    for (int q = 0; q * kTcNT < c; ++q)
-      p.groups[gst[e] + q] = make_int4(p.e_first + e, starts[e] + q * kTcNT, min(kTcNT, c - q * kTcNT), 0);
+    for (int q = 0; (q << p.cap_log2) < c; ++q)
+      p.groups[gst[e] + q] = make_int4(p.e_first + e, starts[e] + (q << p.cap_log2), min(1 << p.cap_log2, c - (q << p.cap_log2)), 0);
     if (has_dup) {   // sequential, stable placement of this expert's slots
       int c2 = starts[e];
       for (int i = 0; i < p.n_slots; ++i)
@@ -472,7 +474,8 @@ inline size_t moe_sort_smem(size_t e_count, size_t T) {
 }
 
 // One warp-iteration = eight 32-blocks of one row (four lanes per block), as quantize_rows_kernel.
-template <class SRC>
+// SPLIT: rows in split form (kdnn_split.cuh) instead of int8 rows.
+template <class SRC, bool SPLIT>
 __device__ void quantize_rows_part(const SRC* src, size_t ld, int nrows, int K, uint8_t* dst,
                                    size_t pitch_bytes, int gwarp, int nwarp) {
   const int nblk = K / 32, per_row = (nblk + 7) / 8;
@@ -489,6 +492,10 @@ __device__ void quantize_rows_part(const SRC* src, size_t ld, int nrows, int K, 
     float d;
     int part, total;
     const uint2 packed = quantize_block_lane8(v, d, part, total);
+    if (SPLIT) {   // K is a multiple of 256: the warp holds one whole super-block
+      split_store_lane8<256>(out, static_cast<size_t>(K), b, packed, d, total);
+      continue;
+    }
     if (b >= nblk) continue;
     reinterpret_cast<uint2*>(out + static_cast<size_t>(b) * 32)[l4] = packed;
     if (l4 == 0) {
@@ -500,29 +507,30 @@ __device__ void quantize_rows_part(const SRC* src, size_t ld, int nrows, int K, 
   }
 }
 
-template <class SRC>
+template <class SRC, bool SPLIT>
 __global__ void __launch_bounds__(1024, 1) moe_prep_kernel(const PrepParams p) {
   pdl_chain_entry();
   extern __shared__ uint32_t prep_smem[];
   if (blockIdx.x == 0) {
     moe_sort_block(p, prep_smem);
   } else if (p.X != nullptr) {
-    quantize_rows_part<SRC>(static_cast<const SRC*>(p.X), p.ldx, p.T, p.H, p.xrows, p.x_pitch,
+    quantize_rows_part<SRC, SPLIT>(static_cast<const SRC*>(p.X), p.ldx, p.T, p.H, p.xrows, p.x_pitch,
                             (blockIdx.x - 1) * (blockDim.x >> 5) + (threadIdx.x >> 5), (gridDim.x - 1) * (blockDim.x >> 5));
   }
 }
 
-static cudaError_t moe_prep_launch(const PrepParams& p, int xs, cudaStream_t st) {
+static cudaError_t moe_prep_launch(const PrepParams& p, int xs, bool split, cudaStream_t st) {
   const size_t smem = moe_sort_smem(p.e_count, p.T);
   int qctas = 0;
   if (p.X != nullptr) {
     const int items = p.T * ((p.H / 32 + 7) / 8);
     qctas = max(1, min(4 * device_sm_count(), (items + 31) / 32));
   }
-  auto kern = xs == KDNN_F32 ? moe_prep_kernel<float> : moe_prep_kernel<__nv_bfloat16>;
+  auto kern = xs == KDNN_F32 ? (split ? moe_prep_kernel<float, true> : moe_prep_kernel<float, false>)
+                             : (split ? moe_prep_kernel<__nv_bfloat16, true> : moe_prep_kernel<__nv_bfloat16, false>);
   if (smem > 48 * 1024) {   // once per device, at the largest size this kernel is ever given (kPrepSmemLimit)
-    static SmemAttrOnce once[2];
-    const cudaError_t e = set_max_smem_once(once[xs == KDNN_F32], kern, 160 * 1024);
+    static SmemAttrOnce once[4];
+    const cudaError_t e = set_max_smem_once(once[2 * (xs == KDNN_F32) + split], kern, 160 * 1024);
     if (e != cudaSuccess) return e;
   }
   return launch_chained(kern, dim3(1 + qctas), dim3(1024), smem, st, p);
@@ -594,15 +602,45 @@ static MoeWs moe_ws_layout(size_t T, size_t S, size_t H, size_t F, size_t n_expe
   w.pos  = o; o += up(T * S * sizeof(int));
   w.groups = o; o += up((n_experts + T * S / kTcNT + 1) * sizeof(int4));
   w.ngroups = o; o += 256;
-  w.xq   = o; o += up(T * max_sz((H / 64) * sizeof(ActItem), act_row_pitch(H)));
+  w.xq   = o; o += up(T * max_sz((H / 64) * sizeof(ActItem), act_row_pitch_max(H)));
   w.act  = o; o += up(T * S * F * sizeof(float));
-  w.actq = o; o += up(T * S * max_sz((F / 64) * sizeof(ActItem), act_row_pitch(F)));
+  w.actq = o; o += up(T * S * max_sz((F / 64) * sizeof(ActItem), act_row_pitch_max(F)));
   w.out  = o; o += up(T * S * H * sizeof(float));
   w.total = o;
   return w;
 }
 size_t moe_workspace_bytes(size_t T, size_t S, size_t H, size_t F, size_t n_experts) {
   return moe_ws_layout(T, S, H, F, n_experts).total;
+}
+
+// The expert feed-forward on the split-fp16 tensor-core kernel (kdnn_split.cuh): gate/up + SwiGLU + quantization of
+// the result, then the down projection, two launches. `groups` hold up to `cap` (32 or 64) activation rows each.
+static cudaError_t moe_tiles_split(const kdnn_b200_weight_table* gate, const kdnn_b200_weight_table* up,
+                                   const kdnn_b200_weight_table* down, size_t n_slots, size_t S, int xs, size_t e_count,
+                                   int cap, const int4* groups, const int* n_groups, const int* list, const uint8_t* xrows,
+                                   uint8_t* arows, float* out, const PeerOut* po, cudaStream_t st) {
+  const size_t H = gate->cols, F = gate->rows;
+  SplitParams g{};
+  cudaError_t err = moe_status_ptr(&g.status);
+  if (err != cudaSuccess) return err;
+  const int max_groups = static_cast<int>(e_count + n_slots / cap);
+  g.maps0 = static_cast<const CUtensorMap*>(gate->tma); g.maps1 = static_cast<const CUtensorMap*>(up->tma);
+  g.N = (int)F; g.K = (int)H; g.tile_rows = 128; g.box_rows = kTcBoxRows; g.boxes = 128 / kTcBoxRows;
+  g.row_units = (int)((F + 127) / 128);
+  g.groups = groups; g.n_groups = n_groups; g.list = list; g.S = (int)S;
+  g.xrows = xrows; g.x_pitch = split_row_pitch(H, 256); g.round_bf16 = xs == KDNN_BF16;
+  g.qdst = arows; g.q_pitch = split_row_pitch(F, 128);
+  SplitParams d = g;
+  d.maps0 = static_cast<const CUtensorMap*>(down->tma); d.maps1 = nullptr;
+  d.N = (int)H; d.K = (int)F; d.row_units = (int)((H + 255) / 256);
+  d.xrows = arows; d.x_pitch = g.q_pitch; d.dst = out; d.ld_dst = H; d.qdst = nullptr;
+  if (po) d.po = *po;
+  if (cap == 32) {
+    err = launch_grouped_split<1, 2, 1, 1, float>(g, max_groups * g.row_units, st);
+    return err != cudaSuccess ? err : launch_grouped_split<0, 2, 1, 2, float>(d, max_groups * d.row_units, st);
+  }
+  err = launch_grouped_split<1, 2, 2, 1, float>(g, max_groups * g.row_units, st);
+  return err != cudaSuccess ? err : launch_grouped_split<0, 2, 2, 2, float>(d, max_groups * d.row_units, st);
 }
 
 // The expert feed-forward between the slot sort and the combine, Q4_K on the tensor cores:
@@ -676,6 +714,16 @@ static bool tc_covers(const kdnn_b200_weight_table* gate, const kdnn_b200_weight
   const size_t H = gate->cols, F = gate->rows;
   return gate->tma != nullptr && up->tma != nullptr && down->tma != nullptr && F % 64 == 0 && H >= 512 && F >= 256;
 }
+// Whether the split-fp16 kernel runs this call: the default selection, with the tables' descriptors at hand. (A single
+// token leaves both tile kernels mostly idle, 44 and 46 us on 128 experts / top-8 / 2048 x 768: it stays on mma.sync,
+// whose products are rounded in the order of the per-row GEMV.)
+static bool split_covers(const kdnn_b200_weight_table* gate, const kdnn_b200_weight_table* up,
+                         const kdnn_b200_weight_table* down) {
+  return tile_kind() == 3 && gate->tma != nullptr && up->tma != nullptr && down->tma != nullptr && gate->cols % 256 == 0 &&
+         gate->rows % 256 == 0;
+}
+// Activation rows per group: 64 once the experts' mean run is longer than 32 (weights are then unpacked half as often).
+static int split_cap(size_t n_slots, size_t n_experts) { return n_slots > 32 * n_experts ? 64 : 32; }
 
 template <class YT>
 static cudaError_t moe_combine_launch(const float* out, const int* pos, const float* wts, size_t T, size_t S, size_t H,
@@ -719,10 +767,17 @@ cudaError_t moe_ffn_launch(const void* X, size_t ldx, size_t T, int xs,
     pp.offs = offs; pp.list = list; pp.pos = pos;
     pp.groups = reinterpret_cast<int4*>(b + L.groups); pp.n_groups = reinterpret_cast<int*>(b + L.ngroups);
     pp.X = e_count > 0 ? X : nullptr; pp.ldx = ldx; pp.T = (int)T; pp.H = (int)H;
-    pp.xrows = b + L.xq; pp.x_pitch = act_row_pitch(H);
-    err = moe_prep_launch(pp, xs, st);
+    const bool split = T > 1 && split_covers(gate, up, down);
+    const int cap = split ? split_cap(n_slots, gate->n_experts) : kTcNT;
+    pp.cap_log2 = cap == 64 ? 6 : 5;
+    pp.xrows = b + L.xq; pp.x_pitch = split ? split_row_pitch(H, 256) : act_row_pitch(H);
+    err = moe_prep_launch(pp, xs, split, st);
     if (err != cudaSuccess) return err;
-    if (e_count > 0) {
+    if (split && e_count > 0) {
+      err = moe_tiles_split(gate, up, down, n_slots, S, xs, e_count, cap, pp.groups, pp.n_groups, list, pp.xrows,
+                            b + L.actq, out, nullptr, st);
+      if (err != cudaSuccess) return err;
+    } else if (e_count > 0) {
       err = moe_tiles_q4k(kind, gate, up, down, T, S, xs, e_first, e_count, b, L, st);
       if (err != cudaSuccess) return err;
     }
@@ -843,7 +898,7 @@ static ExLayout ex_layout(size_t Tl, size_t world, size_t S, size_t H) {
   const size_t T = Tl * world;
   ExLayout L{};
   size_t o = 0;
-  L.xrows = o; o += up(T * act_row_pitch(H));
+  L.xrows = o; o += up(T * act_row_pitch_max(H));
   L.idx   = o; o += up(T * S * sizeof(int32_t));
   L.rel   = o; o += up(T * S * sizeof(int32_t));
   L.wts   = o; o += up(T * S * sizeof(float));
@@ -874,6 +929,8 @@ struct GateParams {
   int* pos;                     // single rank: position of every slot in `list` (the down rows are kept by position)
   int* ticket; uint32_t* epoch; int* status;
   unsigned long long wait_ns;
+  int cap_log2;                 // activation rows per group: 32 or 64
+  int split;                    // rows in split form (kdnn_split.cuh) instead of int8 rows
 };
 
 __device__ __forceinline__ unsigned cluster_cta_rank() {
@@ -1119,6 +1176,12 @@ __global__ void __launch_bounds__(kGateThreads) moe_gate_kernel(const GateParams
       float d;
       int part, total;
       const uint2 packed = quantize_block_lane8(v, d, part, total);
+      if (p.split) {   // H is a multiple of 256: the warp holds one whole super-block
+        for (int r = 0; r < p.world; ++r)
+          split_store_lane8<256>(p.region[r] + p.L.xrows + static_cast<size_t>(p.rank * p.Tl + t_first + tc) * p.x_pitch,
+                                 static_cast<size_t>(p.H), b, packed, d, total);
+        continue;
+      }
       if (b >= nblk) continue;
       const size_t row_off = p.L.xrows + static_cast<size_t>(p.rank * p.Tl + t_first + tc) * p.x_pitch;
       const float ds = __fmul_rn(static_cast<float>(total), d);
@@ -1190,7 +1253,7 @@ __global__ void __launch_bounds__(kGateThreads) moe_gate_kernel(const GateParams
         c = min(max(raw, 0), n_slots);
         cnt[e] = 0;
       }
-      const int gc = (c + kTcNT - 1) / kTcNT;
+      const int gc = (c + (1 << p.cap_log2) - 1) >> p.cap_log2;
       int incl = c, gincl = gc;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -1201,8 +1264,8 @@ __global__ void __launch_bounds__(kGateThreads) moe_gate_kernel(const GateParams
         const int st = run + incl - c, g0 = grun + gincl - gc;
         starts[e] = st;
         p.offs[e] = st;
-        for (int q = 0; q * kTcNT < c; ++q)
-          p.groups[g0 + q] = make_int4(p.e_first + e, st + q * kTcNT, min(kTcNT, c - q * kTcNT), 0);
+        for (int q = 0; (q << p.cap_log2) < c; ++q)
+          p.groups[g0 + q] = make_int4(p.e_first + e, st + (q << p.cap_log2), min(1 << p.cap_log2, c - (q << p.cap_log2)), 0);
       }
       run += __shfl_sync(0xFFFFFFFFu, incl, 31);
       grun += __shfl_sync(0xFFFFFFFFu, gincl, 31);
@@ -1440,7 +1503,7 @@ static BlockWs block_ws_layout(size_t T, size_t S, size_t H, size_t F, size_t n_
   w.groups = o; o += up((n_experts + T * S / kTcNT + 1) * sizeof(int4));
   w.ngroups = o; o += 256;
   w.act  = o; o += up(T * S * F * sizeof(float));
-  w.actq = o; o += up(T * S * act_row_pitch(F));
+  w.actq = o; o += up(T * S * act_row_pitch_max(F));
   w.sync = o; o += 256;          // gate ticket, down ticket, epoch
   w.region = o; o += region_bytes;
   w.total = o;
@@ -1472,7 +1535,10 @@ cudaError_t moe_block_launch(const BlockArgs& a, cudaStream_t st) {
   g.Tl = (int)a.Tl; g.H = (int)H; g.E = (int)E; g.top_k = a.top_k; g.norm_topk = a.norm_topk; g.sigmoid = a.sigmoid;
   g.world = a.world; g.rank = a.rank; g.routed_scale = a.routed_scale;
   for (size_t r = 0; r < world; ++r) g.region[r] = regions[r];
-  g.L = XL; g.x_pitch = act_row_pitch(H);
+  const bool split = split_covers(a.gate, a.up, a.down);
+  const int cap = split ? split_cap(T * S, E) : kTcNT;
+  g.split = split; g.cap_log2 = cap == 64 ? 6 : 5;
+  g.L = XL; g.x_pitch = split ? split_row_pitch(H, 256) : act_row_pitch(H);
   g.e_per_rank = a.world > 1 ? (int)a.e_count : 0; g.e_first = (int)a.e_first; g.e_count = (int)a.e_count;
   g.offs = reinterpret_cast<int*>(b + L.offs); g.list = reinterpret_cast<int*>(b + L.list);
   g.groups = reinterpret_cast<int4*>(b + L.groups); g.n_groups = reinterpret_cast<int*>(b + L.ngroups);
@@ -1512,7 +1578,11 @@ cudaError_t moe_block_launch(const BlockArgs& a, cudaStream_t st) {
   po.world = a.world; po.rank = a.rank;
   po.ticket = a.world > 1 ? sync + 1 : nullptr;
   po.epoch = reinterpret_cast<const uint32_t*>(sync + 2);
-  if (a.e_count > 0) {
+  if (split && a.e_count > 0) {
+    err = moe_tiles_split(a.gate, a.up, a.down, T * S, S, a.scalar, a.e_count, cap, g.groups, g.n_groups, g.list,
+                          mine + XL.xrows, b + L.actq, by_position ? reinterpret_cast<float*>(mine + XL.out) : nullptr, &po, st);
+    if (err != cudaSuccess) return err;
+  } else if (a.e_count > 0) {
     const int want = tile_kind() == 3 ? 1 : tile_kind();
     const int kind = (want == 2 && !tc_covers(a.gate, a.up, a.down)) || want == 0 ? 1 : want;
     const int n_slots = (int)(T * S);

@@ -672,13 +672,13 @@ using TcEncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, v
 TcEncodeFn tc_encode_fn();   // kdnn_moe.cu
 
 // Tensor map of one packed Q4_K matrix: bytes as the inner dimension, rows as the outer, boxes of
-// 32 rows x one 144-byte super-block.
-inline cudaError_t tc_encode_matrix(CUtensorMap* out, const void* w, size_t rows, size_t row_bytes) {
+// `box_rows` rows x one 144-byte super-block.
+inline cudaError_t tc_encode_matrix(CUtensorMap* out, const void* w, size_t rows, size_t row_bytes, int box_rows = kTcBoxRows) {
   TcEncodeFn fn = tc_encode_fn();
   if (fn == nullptr) return cudaErrorNotSupported;
   const cuuint64_t dims[2]    = {static_cast<cuuint64_t>(row_bytes), static_cast<cuuint64_t>(rows)};
   const cuuint64_t strides[1] = {static_cast<cuuint64_t>(row_bytes)};
-  const cuuint32_t box[2]     = {144u, static_cast<cuuint32_t>(kTcBoxRows)};
+  const cuuint32_t box[2]     = {144u, static_cast<cuuint32_t>(box_rows)};
   const cuuint32_t estr[2]    = {1u, 1u};
   const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(w), dims, strides, box, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
