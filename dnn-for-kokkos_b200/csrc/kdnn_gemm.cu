@@ -3,6 +3,7 @@
 // holds all M activation rows. Row m of Y equals the decode GEMV applied to row m.
 #include "kdnn_grouped.cuh"
 #include "kdnn_mma.cuh"
+#include "kdnn_rowmma.cuh"
 #include "kdnn_split.cuh"
 #include "kdnn_tc.cuh"
 
@@ -19,6 +20,7 @@ static size_t gemm_items_offset(size_t M) {
   return gemm_groups_offset(M) + (((M + kTcNT - 1) / kTcNT * sizeof(int4) + 255) & ~size_t(255));
 }
 size_t gemm_workspace_bytes(size_t M, size_t K) {
+  // (rowmma_x_bytes of four rows and more is below the second figure: 10 bytes an element at four rows, 16 there)
   const size_t a = M * (K / 64) * sizeof(ActItem), b = M * act_row_pitch_max(K);
   return gemm_items_offset(M) + (a > b ? a : b);
 }
@@ -80,14 +82,30 @@ static cudaError_t gemm_split(const void* w, size_t N, size_t K, const void* X, 
   return ys == KDNN_F32 ? launch_grouped_split<2, 1, 1, 1, float>(q, units, st) : launch_grouped_split<2, 1, 1, 1, __nv_bfloat16>(q, units, st);
 }
 
+template <uint32_t DT>
+static cudaError_t gemm_rowmma_dt(const RmParams& p, const void* X, size_t ldx, int xs, uint8_t* xrows, cudaStream_t st) {
+  return xs == KDNN_F32 ? launch_rowmma<DT, float>(p, static_cast<const float*>(X), ldx, xrows, st)
+                        : launch_rowmma<DT, __nv_bfloat16>(p, static_cast<const __nv_bfloat16*>(X), ldx, xrows, st);
+}
+static cudaError_t gemm_rowmma(uint32_t dt, const void* w, size_t N, size_t K, const void* X, size_t ldx, size_t M, int xs,
+                               void* Y, size_t ldy, int ys, uint8_t* xrows, cudaStream_t st) {
+  RmParams p{};
+  p.w = static_cast<const uint8_t*>(w);
+  p.row_bytes = row_bytes_of(dt, K); p.total = N * p.row_bytes;
+  p.N = (int)N; p.M = (int)M; p.blocks = (int)(K / 256);
+  p.x = xrows; p.y = Y; p.ldy = ldy; p.y_bf16 = ys == KDNN_BF16;
+  if (dt == KDNN_GGML_Q5_K) return gemm_rowmma_dt<KDNN_GGML_Q5_K>(p, X, ldx, xs, xrows, st);
+  if (dt == KDNN_GGML_Q6_K) return gemm_rowmma_dt<KDNN_GGML_Q6_K>(p, X, ldx, xs, xrows, st);
+  return gemm_rowmma_dt<KDNN_GGML_Q8_0>(p, X, ldx, xs, xrows, st);
+}
+
 // `dots` (parity probe, tcgen05 kernel only): int32 [M][N][K/32] raw sub-block dots, or nullptr.
 cudaError_t gemm_launch(uint32_t dt, const void* w, size_t N, size_t K, const void* X, size_t ldx,
                         size_t M, int xs, void* Y, size_t ldy, int ys, void* ws, int32_t* dots, cudaStream_t st) {
   uint8_t* b      = static_cast<uint8_t*>(ws);
   // Crossover measured on a 14336 x 4096 Q4_K matrix: one GEMV kernel per activation row (6.9 us each) beats
-  // the tile kernels (24 us and up) for up to three rows; the tcgen05 kernel is the faster tile kernel up
-  // to eight rows (24-27 us against 30-31 us), the mma.sync kernel beyond (28 / 37 us against 31 / 42 us
-  // at 16 / 32 rows).
+  // the tile kernels (23 us and up) for up to three rows; above, the split-fp16 kernel is the fastest on Q4_K (23.4 / 27.9 us at
+  // 8 / 32 rows; integer tcgen05 27.4 / 42, mma.sync 30 / 37).
   int kind = tile_kind();
   if (kind == 3 && dots == nullptr) {
     if (M <= 3) {
@@ -102,6 +120,10 @@ cudaError_t gemm_launch(uint32_t dt, const void* w, size_t N, size_t K, const vo
     }
     if (dt == KDNN_GGML_Q4_K && (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && tc_encode_fn() != nullptr)
       return gemm_split(w, N, K, X, ldx, M, xs, Y, ldy, ys, b, st);
+    // Every other format whose rows are whole 256-element groups (Q8_0 rows may not be) and start the matrix on 16 bytes
+    // (its 16-byte copies step back to that boundary): 4096 x 14336 Q6_K, 16 rows 32.3 us, 433 on the dp4a kernel below.
+    if (dt != KDNN_GGML_Q4_K && K % 256 == 0 && (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && rowmma_x_bytes(M, K) <= M * act_row_pitch_max(K))
+      return gemm_rowmma(dt, w, N, K, X, ldx, M, xs, Y, ldy, ys, b + gemm_items_offset(M), st);
     kind = 1;
   } else if (kind == 3) {
     kind = 2;
