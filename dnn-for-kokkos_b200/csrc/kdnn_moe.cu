@@ -715,8 +715,7 @@ static bool tc_covers(const kdnn_b200_weight_table* gate, const kdnn_b200_weight
   return gate->tma != nullptr && up->tma != nullptr && down->tma != nullptr && F % 64 == 0 && H >= 512 && F >= 256;
 }
 // Whether the split-fp16 kernel runs this call: the default selection, with the tables' descriptors at hand. (A single
-// token leaves both tile kernels mostly idle, 44 and 46 us on 128 experts / top-8 / 2048 x 768: it stays on mma.sync,
-// whose products are rounded in the order of the per-row GEMV.)
+// token leaves both tile kernels mostly idle: the token kernels take it, mma.sync where its slots do not fit them.)
 static bool split_covers(const kdnn_b200_weight_table* gate, const kdnn_b200_weight_table* up,
                          const kdnn_b200_weight_table* down) {
   return tile_kind() == 3 && gate->tma != nullptr && up->tma != nullptr && down->tma != nullptr && gate->cols % 256 == 0 &&
@@ -737,6 +736,156 @@ static cudaError_t moe_combine_launch(const float* out, const int* pos, const fl
                         pos, wts, (int)T, (int)S, (int)H, static_cast<YT*>(Y), ldy);
 }
 
+// ---- one token ---------------------------------------------------------------------------------
+// A single token leaves every expert one activation row: nothing to group and nothing for a tile kernel to reuse, so the
+// slot sort, the quantizer launches and the combine are only latency. Two launches take the call: every CTA quantizes what
+// it needs into shared memory itself (a few microseconds of L2 reads less than a launch and its gap), a warp walks one
+// weight row at a time, a lane per 64-element item, with the items of kdnn_tile.cuh, so every format runs here.
+// 128 experts, top-8, 2048 x 768, route and feed-forward: 27.5 us, 45.9 to 48.2 through sort and tiles (packed bytes: 3.2 us);
+// bound by the three dependent launches.
+struct TokenParams {
+  const uintptr_t* w0; const uintptr_t* w1;   // gate and up, or down
+  int row_bytes, N, K;                        // rows and elements a row of these matrices
+  const int32_t* idx; const float* wts;
+  int S, e_first, e_count;
+  const void* x; float* act; void* y;         // x [K] of XT -> act [S][N] (gate/up); act [S][K] -> y [N] (down)
+  int round_bf16, y_bf16;
+};
+
+// Whether slot s counts: an expert of this table range with a weight (as the combine of the general path).
+__device__ __forceinline__ bool token_slot(const TokenParams& p, int s, int& expert) {
+  const int e = p.idx[s] - p.e_first;
+  expert = p.e_first + e;
+  return e >= 0 && e < p.e_count && p.wts[s] != 0.0f;
+}
+
+// n elements (a multiple of 64) into ActItems in shared memory, by the whole CTA.
+template <uint32_t DT, class SRC>
+__device__ __forceinline__ void token_quantize(const SRC* x, int n, ActItem* out) {
+  const int lane = threadIdx.x & 31, l8 = lane & 7, nblk = n / 32;
+  const bool vec_ok = (reinterpret_cast<uintptr_t>(x) & (sizeof(SRC) * 4 - 1)) == 0;
+  for (int base = (threadIdx.x >> 5) * 4; base < nblk; base += (blockDim.x >> 5) * 4) {
+    const int b = base + (lane >> 3);
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    if (b < nblk) load4<SRC>(x, static_cast<size_t>(b) * 32 + l8 * 4, vec_ok, v);
+    float d;
+    int part, total;
+    const uint32_t packed = quantize_block_lane(v, d, part, total);
+    if (b >= nblk) continue;
+    int item, g;
+    granule_map<DT>(b, l8 >> 2, item, g);
+    ActItem& a = out[item];
+    reinterpret_cast<uint32_t*>(&a.g[g])[l8 & 3] = packed;
+    if ((l8 & 3) == 0) { a.dx[g] = d; a.sum[g] = part; }
+  }
+}
+
+constexpr int kTokenWarps = 8, kTokenRows = 2;   // gate/up: rows per warp, so that a CTA's quantized row serves sixteen
+
+template <uint32_t DT, class XT>
+__global__ void __launch_bounds__(32 * kTokenWarps) moe_token_gate_up_kernel(const TokenParams p) {
+  extern __shared__ __align__(16) uint8_t token_smem[];
+  ActItem* items = reinterpret_cast<ActItem*>(token_smem);
+  pdl_chain_entry();
+  int expert;
+  if (!token_slot(p, blockIdx.y, expert)) return;
+  token_quantize<DT, XT>(static_cast<const XT*>(p.x), p.K, items);
+  __syncthreads();
+  const uint8_t* g0 = reinterpret_cast<const uint8_t*>(p.w0[expert]);
+  const uint8_t* u0 = reinterpret_cast<const uint8_t*>(p.w1[expert]);
+  const int lane = threadIdx.x & 31, nitems = p.K / 64;
+  const int j0 = (blockIdx.x * kTokenWarps + (threadIdx.x >> 5)) * kTokenRows;
+  float g[kTokenRows] = {}, u[kTokenRows] = {};
+  for (int i = lane; i < nitems; i += 32) {
+    const ActItem a = lds_item(items + i);
+#pragma unroll
+    for (int r = 0; r < kTokenRows; ++r) {
+      const size_t off = static_cast<size_t>(min(j0 + r, p.N - 1)) * p.row_bytes;
+      WItem<DT> wg, wu;
+      wg.load(g0 + off, i);
+      wu.load(u0 + off, i);
+      g[r] += wg.dot(a);
+      u[r] += wu.dot(a);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < kTokenRows; ++r) {
+    const float gs = warp_sum(g[r]), us = warp_sum(u[r]);
+    float v = (gs / (1.0f + expf(-gs))) * us;
+    if (p.round_bf16) v = __bfloat162float(__float2bfloat16_rn(v));
+    if (lane == 0 && j0 + r < p.N) p.act[static_cast<size_t>(blockIdx.y) * p.N + j0 + r] = v;
+  }
+}
+
+template <uint32_t DT>
+__global__ void __launch_bounds__(32 * kTokenWarps) moe_token_down_kernel(const TokenParams p) {
+  extern __shared__ __align__(16) uint8_t token_smem[];
+  ActItem* items = reinterpret_cast<ActItem*>(token_smem);   // [S][K / 64]
+  pdl_chain_entry();
+  const int nitems = p.K / 64;
+  int expert;
+  for (int s = 0; s < p.S; ++s)
+    if (token_slot(p, s, expert)) token_quantize<DT, float>(p.act + static_cast<size_t>(s) * p.K, p.K, items + s * nitems);
+  __syncthreads();
+  const int lane = threadIdx.x & 31, j = blockIdx.x * kTokenWarps + (threadIdx.x >> 5);
+  if (j >= p.N) return;
+  float acc = 0.f;
+#pragma unroll 4
+  for (int f = lane; f < p.S * nitems; f += 32) {
+    const int s = f / nitems, i = f - s * nitems;
+    if (!token_slot(p, s, expert)) continue;
+    WItem<DT> w;
+    w.load(reinterpret_cast<const uint8_t*>(p.w0[expert]) + static_cast<size_t>(j) * p.row_bytes, i);
+    acc += p.wts[s] * w.dot(lds_item(items + f));
+  }
+  acc = warp_sum(acc);
+  if (lane != 0) return;
+  if (p.y_bf16) store_scalar(static_cast<__nv_bfloat16*>(p.y) + j, acc);
+  else store_scalar(static_cast<float*>(p.y) + j, acc);
+}
+
+constexpr size_t kTokenSmem = 48 * 1024;   // quantized rows of one CTA: what a launch gets without asking
+static bool token_covers(size_t S, size_t H, size_t F) {
+  return H / 64 * sizeof(ActItem) <= kTokenSmem && S * (F / 64) * sizeof(ActItem) <= kTokenSmem && S <= 65535;
+}
+
+template <uint32_t DT>
+static cudaError_t token_gate_up(const TokenParams& p, int xs, cudaStream_t st) {
+  const dim3 grid((p.N + kTokenWarps * kTokenRows - 1) / (kTokenWarps * kTokenRows), p.S);
+  return launch_chained(xs == KDNN_F32 ? moe_token_gate_up_kernel<DT, float> : moe_token_gate_up_kernel<DT, __nv_bfloat16>, grid,
+                        dim3(32 * kTokenWarps), p.K / 64 * sizeof(ActItem), st, p);
+}
+template <uint32_t DT>
+static cudaError_t token_down(const TokenParams& p, cudaStream_t st) {
+  return launch_chained(moe_token_down_kernel<DT>, dim3((p.N + kTokenWarps - 1) / kTokenWarps), dim3(32 * kTokenWarps),
+                        static_cast<size_t>(p.S) * (p.K / 64) * sizeof(ActItem), st, p);
+}
+
+static cudaError_t moe_token_launch(const void* X, int xs, const kdnn_b200_weight_table* gate, const kdnn_b200_weight_table* up,
+                                    const kdnn_b200_weight_table* down, const int32_t* idx, const float* wts, size_t S, void* Y,
+                                    int ys, size_t e_first, size_t e_count, float* act, cudaStream_t st) {
+  TokenParams p{};
+  p.w0 = gate->base; p.w1 = up->base; p.row_bytes = (int)gate->row_bytes; p.N = (int)gate->rows; p.K = (int)gate->cols;
+  p.idx = idx; p.wts = wts; p.S = (int)S; p.e_first = (int)e_first; p.e_count = (int)e_count;
+  p.x = X; p.act = act; p.round_bf16 = xs == KDNN_BF16;
+  cudaError_t e;
+  switch (gate->ggml_type) {
+    case KDNN_GGML_Q4_K: e = token_gate_up<KDNN_GGML_Q4_K>(p, xs, st); break;
+    case KDNN_GGML_Q5_K: e = token_gate_up<KDNN_GGML_Q5_K>(p, xs, st); break;
+    case KDNN_GGML_Q6_K: e = token_gate_up<KDNN_GGML_Q6_K>(p, xs, st); break;
+    default: e = token_gate_up<KDNN_GGML_Q8_0>(p, xs, st); break;
+  }
+  if (e != cudaSuccess) return e;
+  p.w0 = down->base; p.w1 = nullptr; p.row_bytes = (int)down->row_bytes; p.N = (int)down->rows; p.K = (int)down->cols;
+  p.y = Y; p.y_bf16 = ys == KDNN_BF16;
+  switch (down->ggml_type) {
+    case KDNN_GGML_Q4_K: return token_down<KDNN_GGML_Q4_K>(p, st);
+    case KDNN_GGML_Q5_K: return token_down<KDNN_GGML_Q5_K>(p, st);
+    case KDNN_GGML_Q6_K: return token_down<KDNN_GGML_Q6_K>(p, st);
+    default: return token_down<KDNN_GGML_Q8_0>(p, st);
+  }
+}
+
 cudaError_t moe_ffn_launch(const void* X, size_t ldx, size_t T, int xs,
                            const kdnn_b200_weight_table* gate, const kdnn_b200_weight_table* up,
                            const kdnn_b200_weight_table* down, const int32_t* idx, const float* wts,
@@ -753,6 +902,8 @@ cudaError_t moe_ffn_launch(const void* X, size_t ldx, size_t T, int xs,
   ActItem* xq   = reinterpret_cast<ActItem*>(b + L.xq);
   ActItem* actq = reinterpret_cast<ActItem*>(b + L.actq);
   float* out = reinterpret_cast<float*>(b + L.out);
+  if (T == 1 && tile_kind() == 3 && token_covers(S, H, F))
+    return moe_token_launch(X, xs, gate, up, down, idx, wts, S, Y, ys, e_first, e_count, act, st);
   const int n_slots = static_cast<int>(T * S);
   const bool all_q4k = gate->ggml_type == KDNN_GGML_Q4_K && down->ggml_type == KDNN_GGML_Q4_K &&
                        (reinterpret_cast<uintptr_t>(ws) & 15u) == 0;
