@@ -74,3 +74,21 @@ def test_argument_errors(kd):
         kd.dequant_to_dense(kd.QuantWeight(w.data, 99, 4, 512), torch.empty((4, 512), dtype=torch.float32, device="cuda:0"))
     empty = kd.QuantWeight(torch.empty(0, dtype=torch.uint8, device="cuda:0"), O.Q4_K, 0, 512)
     kd.dequant_to_dense(empty, torch.empty((0, 512), dtype=torch.float32, device="cuda:0"))   # no launch, no error
+
+
+@pytest.mark.parametrize("dtype", TYPES)
+@pytest.mark.parametrize("out", [torch.float32, torch.bfloat16])
+def test_wide_loads_equal_byte_loads(kd, dtype, out):
+    """A matrix on its natural boundary takes wide loads, the same bytes one place further take byte loads: same bits."""
+    rows, cols = 5, 768
+    packed = torch.from_numpy(np.ascontiguousarray(_payload(kd, dtype, rows, cols, 9)).reshape(-1).copy())
+    big = torch.zeros(packed.numel() + 17, dtype=torch.uint8, device="cuda:0")
+    got = []
+    for shift in (0, 1):
+        big[shift:shift + packed.numel()] = packed.to("cuda:0")
+        Y = torch.full((rows, cols), float("nan"), dtype=out, device="cuda:0")
+        torch.cuda.synchronize()
+        kd.dequant_to_dense(kd.QuantWeight(big[shift:shift + packed.numel()], dtype, rows, cols), Y)
+        torch.cuda.synchronize()
+        got.append(Y.float().cpu().numpy().view(np.uint32))
+    assert np.array_equal(got[0], got[1])
