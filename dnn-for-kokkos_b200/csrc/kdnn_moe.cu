@@ -1032,7 +1032,8 @@ cudaError_t residual_rmsnorm_launch(const void* h, size_t ldh, const float* y, s
 //   4. moe_combine_norm_kernel   waits for every rank's flag, sums the slots in slot order, adds the
 //                          residual and forms the next block's un-scaled RMS norm
 // Exchange region of one rank (all ranks use the same layout; T = tokens_local * world):
-//   xrows  [T] quantized token rows        written by every rank's gate kernel (its own tokens)
+//   xrows  [T] quantized token rows        written by every rank's gate kernel (its own tokens); with several ranks
+//                                          always int8 rows (act_row_pitch), the form every rank can read
 //   idx    [T][S] routed expert ids        written by every rank's gate kernel (its own tokens)
 //   rel    [T][S] rank of the slot inside its expert's run on the expert's owner (only the owner's copy
 //                 of a slot's entry is written)
@@ -1049,7 +1050,7 @@ static ExLayout ex_layout(size_t Tl, size_t world, size_t S, size_t H) {
   const size_t T = Tl * world;
   ExLayout L{};
   size_t o = 0;
-  L.xrows = o; o += up(T * act_row_pitch_max(H));
+  L.xrows = o; o += up(T * (world > 1 ? act_row_pitch(H) : act_row_pitch_max(H)));   // what travels is int8 rows
   L.idx   = o; o += up(T * S * sizeof(int32_t));
   L.rel   = o; o += up(T * S * sizeof(int32_t));
   L.wts   = o; o += up(T * S * sizeof(float));
@@ -1081,7 +1082,7 @@ struct GateParams {
   int* ticket; uint32_t* epoch; int* status;
   unsigned long long wait_ns;
   int cap_log2;                 // activation rows per group: 32 or 64
-  int split;                    // rows in split form (kdnn_split.cuh) instead of int8 rows
+  int split;                    // rows in split form (kdnn_split.cuh) instead of int8 rows (world == 1)
 };
 
 __device__ __forceinline__ unsigned cluster_cta_rank() {
@@ -1327,10 +1328,9 @@ __global__ void __launch_bounds__(kGateThreads) moe_gate_kernel(const GateParams
       float d;
       int part, total;
       const uint2 packed = quantize_block_lane8(v, d, part, total);
-      if (p.split) {   // H is a multiple of 256: the warp holds one whole super-block
-        for (int r = 0; r < p.world; ++r)
-          split_store_lane8<256>(p.region[r] + p.L.xrows + static_cast<size_t>(p.rank * p.Tl + t_first + tc) * p.x_pitch,
-                                 static_cast<size_t>(p.H), b, packed, d, total);
+      if (p.split) {   // one rank only; H is a multiple of 256: the warp holds one whole super-block
+        split_store_lane8<256>(p.region[0] + p.L.xrows + static_cast<size_t>(t_first + tc) * p.x_pitch,
+                               static_cast<size_t>(p.H), b, packed, d, total);
         continue;
       }
       if (b >= nblk) continue;
@@ -1686,7 +1686,9 @@ cudaError_t moe_block_launch(const BlockArgs& a, cudaStream_t st) {
   g.Tl = (int)a.Tl; g.H = (int)H; g.E = (int)E; g.top_k = a.top_k; g.norm_topk = a.norm_topk; g.sigmoid = a.sigmoid;
   g.world = a.world; g.rank = a.rank; g.routed_scale = a.routed_scale;
   for (size_t r = 0; r < world; ++r) g.region[r] = regions[r];
-  const bool split = split_covers(a.gate, a.up, a.down);
+  // Rows that travel are int8 rows whatever this rank's tables and tile kind are: a peer reads them in ITS form, and all
+  // integer kernels share that one (3968 bytes a row at hidden 2048, the split form 8480).
+  const bool split = a.world == 1 && split_covers(a.gate, a.up, a.down);
   const int cap = split ? split_cap(T * S, E) : kTcNT;
   g.split = split; g.cap_log2 = cap == 64 ? 6 : 5;
   g.L = XL; g.x_pitch = split ? split_row_pitch(H, 256) : act_row_pitch(H);

@@ -273,8 +273,10 @@ def check_multi_rank(kd, dev, rank: int, world: int, layers: int = 2, cfg: Optio
     g = torch.Generator(device=dev).manual_seed(cfg.seed)
     h0 = torch.randn(cfg.tokens, cfg.hidden, device=dev, generator=g).to(torch.bfloat16)
     out = {}
+    prev_kind = kd.tile_kind(1)    # the kernel a block of several ranks runs on: the same roundings on both sides
     single = MoeStack(kd, dev, cfg, 0, 1, exchange="push").forward(h0).float()
     torch.cuda.synchronize()
+    kd.tile_kind(prev_kind)
     for mode in ("push", "allreduce"):
         if world > 1:
             dist.barrier()

@@ -279,7 +279,8 @@ int kdnn_b200_moe_ffn(const void* X, size_t ldx, size_t T, int x_scalar,
  * kdnn_b200_moe_exchange_bytes() that ALL ranks can address (cudaMalloc + cudaIpc handles, or any other
  * peer-mapped allocation; zero it once before the first call). `regions[r]` is rank r's region as seen from
  * THIS process; regions[rank] is the local one. Every rank makes the same sequence of block calls with the
- * same tokens_local, world, top_k and hidden size. No counterpart in the reference, which is single-device
+ * same tokens_local, world, top_k and hidden size; tables with or without TMA descriptors and the tile kind may
+ * differ between the ranks (the rows that travel have one form). No counterpart in the reference, which is single-device
  * (there is no collective anywhere in it); the partition rule is expert e on rank e / (E / world). */
 typedef struct {
   int rank, world;            /* world <= 8 */

@@ -102,6 +102,24 @@ def test_invalid_arguments_raise(kd):
     kd.moe_route(torch.zeros(0, 4), None, 2, True, 1.0, torch.zeros(0, 2, dtype=torch.int32), torch.zeros(0, 2))
 
 
+def _up(v):
+    return (v + 255) // 256 * 256
+
+
+def _int8_row(K):
+    """Bytes between quantized int8 rows: int8, 16-byte headers, {d, d * sum} and three bf16 parts per 32 elements."""
+    return _up(K + 16 * (K // 32) + 8 * (K // 32) + 48 * ((K // 32 + 7) // 8))
+
+
+@pytest.mark.parametrize("H", [256, 2048, 4096])
+def test_exchange_region_of_several_ranks_holds_int8_rows(kd, H):
+    """What travels between ranks does not depend on the kernels a rank prefers: int8 rows, routing, down rows."""
+    for Tl, world, S in ((1, 2, 1), (3, 2, 2), (32, 8, 8)):
+        T = Tl * world
+        want = _up(T * _int8_row(H)) + 3 * _up(T * S * 4) + _up(T * S * H * 4) + _up(4096 * 4) + 512
+        assert kd.MoeExchange.region_bytes(Tl, world, S, H) == want
+
+
 def test_encoders_round_trip(kd, port):
     import numpy as np
     from oracle import oracle as O

@@ -124,6 +124,36 @@ def test_peer_that_never_signals_ends_in_a_status_not_a_hang(kd):
     assert kd.device_status() == 0 and bool(torch.isfinite(y).all())
 
 
+def test_exchanged_rows_do_not_depend_on_this_ranks_tables_or_tile_kind(kd):
+    """What rank 0 of 2 writes into its peer's region is the same bytes with and without TMA descriptors and for every
+    tile kind, because the peer reads it in a form chosen on ITS side. (One token: no order of counters to differ.)"""
+    E, k, H, F = 4, 2, 512, 256
+    tabs = _tables(kd, *_experts(kd, E, H, F, 22), H, F)
+    x = torch.randn(1, H, generator=torch.Generator().manual_seed(3)).to(DEV)
+    rw = torch.randn(E, H, generator=torch.Generator().manual_seed(4)).to(DEV)
+    seen = []
+    for kind, tma in ((3, True), (3, False), (2, True), (1, True)):
+        if not tma:
+            for t in tabs:
+                t.tma = None
+        bufs = [torch.zeros(kd.MoeExchange.region_bytes(1, 2, k, H), dtype=torch.uint8, device=DEV) for _ in range(2)]
+        ex = kd.MoeExchange.local(0, 2, bufs, wait_ns=20_000_000)
+        ws = torch.zeros(kd.moe_block_workspace_bytes(1, 2, k, H, F, E, False), dtype=torch.uint8, device=DEV)
+        y = torch.zeros((1, H), dtype=torch.float32, device=DEV)
+        prev = kd.tile_kind(kind)
+        try:
+            kd.moe_block(x, rw, None, k, True, 1.0, *tabs, ws, y=y, expert_first=0, expert_count=2, exchange=ex)
+            torch.cuda.synchronize()
+        finally:
+            kd.tile_kind(prev)
+        assert kd.device_status() == kd.KDNN_ERR_DEVICE_WAIT     # nobody runs rank 1
+        seen.append(bufs[1].cpu())
+        for t in tabs:
+            t.tma = kd.encode_table_tma(t.base, t.dtype, t.rows, t.cols)
+    assert int(seen[0].count_nonzero()) > H // 2
+    assert all(torch.equal(seen[0], s) for s in seen[1:])
+
+
 # ---- the reference's small MoE operators (tests/Test_MoE.cpp:201-341) -------------------------------
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_small_moe_operators(kd, dtype):
