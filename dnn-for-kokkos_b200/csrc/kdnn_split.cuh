@@ -4,17 +4,21 @@
 //
 //   dst[pos, j] = sum_k W_g[j, k] * x[row(pos), k],  x = the reference's per-32 int8 activations q * d
 //
-// Numerics. Inside a 256-element super-block the weight is d * (sc * q) - dmin * mn with sc * q <= 63 * 15 an integer
-// that fp16 holds exactly, so A = sc * q needs no rounding and no rescale per 32 elements. The activation row is
-// written once (split_store_lane8) as two fp16 parts of  v = q * (16 * d / D),  D the largest d of a G-element
-// group (G = 256 or 128), so |v| <= 2032:  hi = v rounded to a multiple of u (of its own fp16 step where that is
-// coarser), and mid = fp16(v - hi). The products of A and hi are multiples of u, so the fp32 accumulation of a group is
-// exact while the sum stays below 2^24 u; u is the finest of 1/8 .. 1 that leaves one and a half standard deviations of
-// the sum (about 400 |v|_2) below that. mid carries the next eleven bits, and what it loses goes into the next element
-// (sc * q has a large mean that the min term takes off again, so the error of a plain sum counts most).
-// hi and mid are separate accumulator columns, the min term sum mn * (d * block sum) is a third product of K = 16. The drain adds
-//   acc += (D / 16) * (d_w * (P_hi + P_mid) - dmin_w * P_min)
-// in fp32 once per group instead of once per 32 elements.
+// Numerics. Inside a 256-element super-block the weight is d * (sc * q) - dmin * mn, 6-bit sc and 4-bit q. The tensor core
+// accumulates in fp32 and TRUNCATES, so what it sums has to be exact or small beside the result:
+//   * A = sc * q - t is an integer that fp16 holds exactly (t = 8 sc, or the nearest number to it that lets one fp16 fma
+//     form A): weights around zero, so that activations of one sign do not build a large sum that the min term takes off again;
+//   * the rest of the weight is one number per 32 elements, c = d * t - dmin * mn, formed in fp32 and multiplied with the
+//     block's activation sum in a product of its own: c relative to a power of two e as two fp16 parts, the sum as two;
+//   * the activation row is written once (split_store_lane8) as two fp16 parts of  v = q * (256 * d / D),  D the largest d
+//     of a G-element group (G = 256 or 128), so |v| <= 32512. hi is v rounded to a multiple of u: the products of A and hi are
+//     multiples of u and their sum is exact below 2^24 u; u is the power of two that leaves two to three standard
+//     deviations of the sum (230 |v|_2 and less), and the mean that A still has, below that. In a block far below the largest one hi
+//     is rounded to eleven bits of that block instead (the products stay small beside the sum if the large block's weights
+//     count, and exact if they do not). mid = fp16(v - hi) carries the next eleven bits.
+// hi, mid and the block sums have accumulator columns of their own. The drain adds, in fp32 and once per group,
+//   acc += D * (d / 256 * (P_hi + P_mid) + e / 16 * P_c)
+// Error against float64 (relative 2-norm, 2048 x 4096, 24 rows): see tests/test_split_tiles_gpu.py for the bounds by distribution.
 //
 // What bounds it: the per-32 rescale of the integer path (kdnn_mma.cuh, kdnn_tc.cuh) costs two to three instructions
 // per (row, activation row, 32 elements); here the work per weight is the unpack, nine instructions per eight weights
@@ -47,13 +51,14 @@ namespace kdnn {
 
 constexpr int kSpThreads = 28 * 32;
 constexpr int kSpWarpMma = 24, kSpWarpW = 25, kSpWarpX = 26;
-constexpr uint32_t kSpTmemA = 192, kSpTmemMn = 448;   // D: 2 x 96 columns, A: 2 tile parities x 128, mins: 2 x 8
+constexpr uint32_t kSpTmemA = 192, kSpTmemC = 448;    // D: 2 x 96 columns, A: 2 tile parities x 128, c: 2 x 16
 constexpr int kSpExPitch = 132;                       // floats per activation row of the exchange tile (128 rows + pad)
 
 // ---- split activation rows -------------------------------------------------------------------------
 // Per super-block 1024 bytes: 256 fp16 hi, 256 fp16 mid (element order 0 2 1 3 inside every four, the order the
-// nibble unpack produces); then per group of G elements 32 bytes: fp16 (block sum * 16 d / D) of the super-block's
-// eight blocks as 8 high and 8 low parts (blocks outside the group are zero); then D / 16 per group as float.
+// nibble unpack produces); then per group of G elements 32 bytes: fp16 (block sum * 16 d / D) of the group's
+// blocks in high and low parts, per two blocks {high, high, low, low}, twice over when the group has four blocks (the
+// operand beside the high and the low parts of c); then D per group as float.
 __host__ __device__ inline size_t split_sums_offset(size_t K) { return K * 4; }
 __host__ __device__ inline size_t split_scale_offset(size_t K, int G) { return K * 4 + K / G * 32; }
 inline size_t split_row_pitch(size_t K, int G) { return (split_scale_offset(K, G) + K / G * 4 + 255) & ~size_t(255); }
@@ -74,43 +79,44 @@ __device__ __forceinline__ void split_store_lane8(uint8_t* row, size_t K, int b,
   float dm = fmaxf(d, __shfl_xor_sync(0xffffffffu, d, 4));
   dm = fmaxf(dm, __shfl_xor_sync(0xffffffffu, dm, 8));
   if (G == 256) dm = fmaxf(dm, __shfl_xor_sync(0xffffffffu, dm, 16));
-  const float r16 = dm > 0.0f ? 16.0f * __fdiv_rn(d, dm) : 0.0f;
-  float v[8], n2 = 0.0f;
+  const float r = dm > 0.0f ? 256.0f * __fdiv_rn(d, dm) : 0.0f;
+  const float sum = __fmul_rn(static_cast<float>(total), 0.0625f * r);   // at most 65024 in size
+  float v[8], n2 = 0.0f, s1 = fabsf(sum);
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int q = static_cast<int8_t>(((i < 4 ? packed.x : packed.y) >> (8 * (i & 3))) & 0xFFu);
-    v[i] = __fmul_rn(static_cast<float>(q), r16);
+    v[i] = __fmul_rn(static_cast<float>(q), r);
     n2 += v[i] * v[i];
   }
 #pragma unroll
-  for (int o = 1; o < G / 8; o <<= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);   // |v|^2 of the group
-  // 600 |v| <= 2^24 u
-  const float u  = n2 <= 3495.0f * 3495.0f ? 0.125f : n2 <= 6990.0f * 6990.0f ? 0.25f : n2 <= 13981.0f * 13981.0f ? 0.5f : 1.0f;
-  const float ru = n2 <= 3495.0f * 3495.0f ? 8.0f : n2 <= 6990.0f * 6990.0f ? 4.0f : n2 <= 13981.0f * 13981.0f ? 2.0f : 1.0f;
+  for (int o = 1; o < G / 8; o <<= 1) {
+    n2 += __shfl_xor_sync(0xffffffffu, n2, o);                        // |v|^2 of the group
+    if (o >= 4) s1 += __shfl_xor_sync(0xffffffffu, s1, o);            // its blocks' |sum|
+  }
+  // u: the power of two at or above max(600 |v|, 96 sum of |block sums of v|) / 2^24, from 2 to 32
+  const float need = fminf(fmaxf(fmaxf(600.0f * sqrtf(n2), 1536.0f * s1) * 0x1p-24f, 2.0f), 32.0f);
+  const float u = __uint_as_float((__float_as_uint(need) + 0x7FFFFFu) & 0x7F800000u);
+  // this block's own step: its largest |v|, 127 * r, is 1016 to 2032 of them (2^-24 is fp16's last bit)
+  const float own = fmaxf(__uint_as_float(__float_as_uint(r) & 0x7F800000u) * 0.125f, 0x1p-24f);
+  const float step = fminf(u, own), rstep = __uint_as_float(0x7F000000u - __float_as_uint(step));
   __half hi[8], mid[8];
-  float carry = 0.0f;   // what the elements before this one lost: weights are all of one sign before their min is taken off
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    hi[i] = __float2half_rn(rintf(v[i] * ru) * u);
-    const float r = (v[i] - __half2float(hi[i])) + carry;
-    mid[i] = __float2half_rn(r);
-    carry = r - __half2float(mid[i]);
+    hi[i] = __float2half_rn(rintf(v[i] * rstep) * step);
+    mid[i] = __float2half_rn(v[i] - __half2float(hi[i]));
   }
   uint8_t* o = row + static_cast<size_t>(sb) * 1024 + blk * 64 + l4 * 16;
   *reinterpret_cast<uint4*>(o) = make_uint4(pack_half2(hi[0], hi[2]), pack_half2(hi[1], hi[3]), pack_half2(hi[4], hi[6]), pack_half2(hi[5], hi[7]));
   *reinterpret_cast<uint4*>(o + 512) = make_uint4(pack_half2(mid[0], mid[2]), pack_half2(mid[1], mid[3]), pack_half2(mid[4], mid[6]), pack_half2(mid[5], mid[7]));
   const int grp = G == 256 ? sb : 2 * sb + (blk >> 2);
   __half* sums = reinterpret_cast<__half*>(row + split_sums_offset(K)) + static_cast<size_t>(grp) * 16;
-  if (l4 == 0) {
-    const float s = __fmul_rn(static_cast<float>(total), r16);
-    const __half h = __float2half_rn(s);
-    sums[blk] = h;
-    sums[8 + blk] = __float2half_rn(s - __half2float(h));
-  } else if (G == 128 && l4 == 1) {
-    sums[blk ^ 4] = __float2half_rn(0.0f);
-    sums[8 + (blk ^ 4)] = __float2half_rn(0.0f);
+  if (l4 < (G == 256 ? 1 : 2)) {
+    __half* mine = sums + (G == 256 ? blk >> 1 : 2 * l4 + ((blk >> 1) & 1)) * 4 + (blk & 1);
+    const __half h = __float2half_rn(sum);
+    mine[0] = h;
+    mine[2] = __float2half_rn(sum - __half2float(h));
   } else if (l4 == 2 && (blk & (G / 32 - 1)) == 0) {
-    reinterpret_cast<float*>(row + split_scale_offset(K, G))[grp] = dm * 0.0625f;
+    reinterpret_cast<float*>(row + split_scale_offset(K, G))[grp] = dm;
   }
 }
 
@@ -187,7 +193,7 @@ struct SpLayout {
   static constexpr uint32_t b = 0;
   static constexpr uint32_t w = b + kB * kBStage;
   static constexpr uint32_t sums = w + kW * kWStage;
-  static constexpr uint32_t dd = sums + kB * kSStage;       // [4 tiles][128 rows] {d, dmin}
+  static constexpr uint32_t dd = sums + kB * kSStage;       // [4 tiles][128 rows] {d / 256, e / 16}
   static constexpr uint32_t ex = dd + 4 * 128 * 8;          // MODE 1: [NH][gate, up][kExRows][kSpExPitch] float; PAIR 1: [32][kSpExPitch]
   static constexpr int kExRows = 16 / NH;
   static constexpr uint32_t rowp = ex + (kEx ? 32 * kSpExPitch * 4 : 0);
@@ -222,8 +228,12 @@ __device__ __forceinline__ void sp_st32(uint32_t t, const uint32_t (&v)[32]) {
       "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
       : "memory");
 }
-__device__ __forceinline__ void sp_st8(uint32_t t, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%1,%2,%3,%4};" ::"r"(t), "r"(a), "r"(b), "r"(c), "r"(d)
+// two and four words, each twice
+__device__ __forceinline__ void sp_st2x2(uint32_t t, uint32_t a, uint32_t b) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%1,%2,%2};" ::"r"(t), "r"(a), "r"(b) : "memory");
+}
+__device__ __forceinline__ void sp_st4x2(uint32_t t, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%1,%2,%2,%3,%3,%4,%4};" ::"r"(t), "r"(a), "r"(b), "r"(c), "r"(d)
                : "memory");
 }
 __device__ __forceinline__ void sp_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
@@ -248,13 +258,13 @@ __device__ __forceinline__ uint32_t h2_sub(uint32_t a, uint32_t b) {
   return d;
 }
 constexpr uint32_t kH2Magic = 0x64006400u;   // {1024, 1024}: the low four mantissa bits count units, the next four sixteens
-// 64 elements (32 bytes: low nibbles = one sub-block, high nibbles = the next) -> 32 words of sc * q pairs:
-// (1024 + q) * sc - 1024 * sc and (1024 + 16 q) * (sc / 16) - 64 * sc, exact in one fp16 fma each.
+// 64 elements (32 bytes: low nibbles = one sub-block, high nibbles = the next) -> 32 words of pairs sc * q - t, each in one
+// exact fp16 fma: (1024 + q) * sc - fp16(1032 sc), an integer of at most 520, and (1024 + 16 q) * (sc / 16) - 72 sc.
 __device__ __forceinline__ void sp_unpack64(const uint4& a, const uint4& b, uint32_t sc_pair4, int j, uint32_t (&o)[32]) {
   const uint32_t s0 = h2_sub(__byte_perm(sc_pair4, 0x64646464u, 0x4040u + 0x0101u * j), kH2Magic);
   const uint32_t s1 = h2_sub(__byte_perm(sc_pair4, 0x64646464u, 0x4040u + 0x0101u * (j + 1)), kH2Magic);
-  const uint32_t c0 = h2_mul(s0, 0xE400E400u);      // -1024 * sc
-  const uint32_t c1 = h2_mul(s1, 0xD400D400u);      // -64 * sc'
+  const uint32_t c0 = h2_mul(s0, 0xE408E408u);      // -1032 * sc, rounded
+  const uint32_t c1 = h2_mul(s1, 0xD480D480u);      // -72 * sc'
   const uint32_t s1d = h2_mul(s1, 0x2C002C00u);     // sc' / 16
   const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
@@ -266,16 +276,32 @@ __device__ __forceinline__ void sp_unpack64(const uint4& a, const uint4& b, uint
     o[16 + 2 * i + 1] = h2_fma((u & 0x00F000F0u) | kH2Magic, s1d, c1);
   }
 }
+__device__ __forceinline__ float2 h2_to_f2(uint32_t h) { return __half22float2(*reinterpret_cast<const __half2*>(&h)); }
+__device__ __forceinline__ uint32_t f2_to_h2(float2 f) {
+  const __half2 h = __float22half2_rn(f);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+// c / e of the same two sub-blocks in two fp16 parts; nd = -d / e, ndm = -dmin / e. -t is what the fma above leaves for q = 0.
+template <int J>
+__device__ __forceinline__ void sp_offsets(uint32_t sc_pair4, uint32_t mn_pair4, float2 nd, float2 ndm, uint32_t& hi, uint32_t& lo) {
+  const uint32_t sc = h2_sub(__byte_perm(sc_pair4, 0x64646464u, J == 0 ? 0x4140u : 0x4342u), kH2Magic);
+  const uint32_t mn = h2_sub(__byte_perm(mn_pair4, 0x64646464u, J == 0 ? 0x4140u : 0x4342u), kH2Magic);
+  const uint32_t nt = h2_fma(sc, 0x00006400u, h2_mul(sc, 0xC800E408u));   // {1024 sc - fp16(1032 sc), -8 sc'}
+  const float2 c = ffma2(ndm, h2_to_f2(mn), fmul2(nd, h2_to_f2(nt)));
+  hi = f2_to_h2(c);
+  const float2 h = h2_to_f2(hi);
+  lo = f2_to_h2(fadd2(c, make_float2(-h.x, -h.y)));
+}
 
-// Eight activation rows of one TMEM lane, one group of K: acc += s * (d * (hi + mid) - dmin * min).
-__device__ __forceinline__ void sp_fold8(float* acc, const int (&p)[16], const int (&m)[8], const float* scale, float2 d2, float2 nd2) {
+// Eight activation rows of one TMEM lane, one group of K: acc += D * (d * (hi + mid) + e * c).
+__device__ __forceinline__ void sp_fold8(float* acc, const int (&p)[16], const int (&m)[8], const float* scale, float2 d2, float2 e2) {
   const float4 s0 = *reinterpret_cast<const float4*>(scale), s1 = *reinterpret_cast<const float4*>(scale + 4);
   const float2 s[4] = {make_float2(s0.x, s0.y), make_float2(s0.z, s0.w), make_float2(s1.x, s1.y), make_float2(s1.z, s1.w)};
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     float2 t = fadd2(make_float2(__int_as_float(p[2 * i]), __int_as_float(p[2 * i + 1])),
                      make_float2(__int_as_float(p[8 + 2 * i]), __int_as_float(p[9 + 2 * i])));
-    t = ffma2(nd2, make_float2(__int_as_float(m[2 * i]), __int_as_float(m[2 * i + 1])), fmul2(d2, t));
+    t = ffma2(e2, make_float2(__int_as_float(m[2 * i]), __int_as_float(m[2 * i + 1])), fmul2(d2, t));
     const float2 r = ffma2(s[i], t, make_float2(acc[2 * i], acc[2 * i + 1]));
     acc[2 * i] = r.x;
     acc[2 * i + 1] = r.y;
@@ -288,14 +314,15 @@ __device__ __forceinline__ bool sp_elect() {
   return r != 0;
 }
 // The products of one group of K (256 / KH elements of a tile) with 8 * n8 activation rows: the MMAs for hi and mid,
-// then the min product. bk: the group's activation operand, ms: its block sums.
+// then c: its high and low parts in turn, or (KH = 2) both for the group's four blocks. bk: the group's activation operand, ms: its block sums.
 template <int KH, uint32_t BK>
-__device__ __forceinline__ void sp_group(uint32_t td, uint32_t ta, uint32_t tm, uint32_t bk, uint32_t ms, int n8) {
+__device__ __forceinline__ void sp_group(uint32_t td, uint32_t ta, uint32_t tc, uint32_t bk, uint32_t ms, int n8) {
   const uint64_t bd = sp_desc_sw128(bk);
   const uint32_t id = sp_idesc(16 * n8);
 #pragma unroll
   for (int j = 0; j < 16 / KH; ++j) sp_mma(td, ta + 8 * j, bd + (((j >> 2) * BK + (j & 3) * 32) >> 4), id, j != 0);
-  sp_mma(td + 64, tm, tc_desc(ms), sp_idesc((8 * n8 + 15) & ~15), 0u);
+  sp_mma(td + 64, tc, tc_desc(ms), sp_idesc((8 * n8 + 15) & ~15), 0u);
+  if (KH == 1) sp_mma(td + 64, tc + 8, tc_desc(ms), sp_idesc((8 * n8 + 15) & ~15), 1u);
 }
 
 // MODE 0: dst[pos, j] = W0[j,:] . x[pos,:]                               (down projection)
@@ -308,7 +335,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) grouped_split_q4k_kernel(const 
   static_assert(PAIR == 2 || NH == 1, "one row tile: up to 32 activation rows");
   using L = SpLayout<MODE, PAIR, NH, KH>;
   constexpr int kW = L::kW, kB = L::kB, kNT = L::kNT, G = 256 / KH;
-  constexpr int kU = 4 / NH, kD = 2 * NH;      // unpack and drain warpgroups
+  constexpr int kU = 4 / NH;                   // unpack warpgroups; drain: 2 NH
   extern __shared__ __align__(1024) uint8_t sp_smem_raw[];
   const uint32_t base = (smem_u32(sp_smem_raw) + 1023u) & ~1023u;
   uint8_t* smem = sp_smem_raw + (base - smem_u32(sp_smem_raw));
@@ -386,7 +413,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) grouped_split_q4k_kernel(const 
     const int g_lo = kU == 4 ? (warp >> 3) * 2 : 0, g_hi = kU == 4 ? g_lo + 2 : 4;   // 64-element groups of the super-block
     const bool live = q * 32 < p.tile_rows;     // warps past the tile's rows only keep the barriers moving
     const uint32_t ta = tmem + (static_cast<uint32_t>(q * 32) << 16) + kSpTmemA + par * 128;
-    const uint32_t tm = tmem + (static_cast<uint32_t>(q * 32) << 16) + kSpTmemMn + par * 8;
+    const uint32_t tc = tmem + (static_cast<uint32_t>(q * 32) << 16) + kSpTmemC + par * 16;
     const int total = my_units * tiles_u;
     int s = par;
     uint32_t ph = 0, k = 0;                      // weight stage and its phase; this parity's tile count
@@ -395,7 +422,8 @@ __global__ void __launch_bounds__(kSpThreads, 1) grouped_split_q4k_kernel(const 
       const uint8_t* mine = smem + L::w + s * L::kWStage + row * 144;
       const uint4 hdr = *reinterpret_cast<const uint4*>(mine);
       uint4 qa = *reinterpret_cast<const uint4*>(mine + 16 + 32 * g_lo), qb = *reinterpret_cast<const uint4*>(mine + 32 + 32 * g_lo);
-      const uint32_t sc[2] = {hdr.y & 0x3F3F3F3Fu, (hdr.w & 0x0F0F0F0Fu) | ((hdr.y >> 2) & 0x30303030u)};
+      // scales and mins of this warp's sub-blocks: four of the eight when there are four warpgroups
+      const uint32_t sc_lo = hdr.y & 0x3F3F3F3Fu, sc_hi = (hdr.w & 0x0F0F0F0Fu) | ((hdr.y >> 2) & 0x30303030u);
 #pragma unroll 1
       for (int g = g_lo; g < g_hi; ++g) {
         const uint4 ca = qa, cb = qb;
@@ -404,19 +432,41 @@ __global__ void __launch_bounds__(kSpThreads, 1) grouped_split_q4k_kernel(const 
           qb = *reinterpret_cast<const uint4*>(mine + 64 + 32 * g);
         }
         uint32_t o[32];
-        if (live) sp_unpack64(ca, cb, g < 2 ? sc[0] : sc[1], 2 * (g & 1), o);
+        if (live) sp_unpack64(ca, cb, g < 2 ? sc_lo : sc_hi, 2 * (g & 1), o);
         if (g == g_lo) {   // (the first group is formed while the previous tile's MMAs still read the buffer)
           if (!wait(a_empty(par), (k & 1u) ^ 1u)) { ok = false; break; }
           tc_after();
         }
-        if (live) sp_st32(ta + 32 * g, o);
+        if (live) {
+          sp_st32(ta + 32 * g, o);
+        }
       }
       if (!ok) break;
-      if (g_lo == 0 && live) {
-        const uint32_t mn[2] = {hdr.z & 0x3F3F3F3Fu, ((hdr.w >> 4) & 0x0F0F0F0Fu) | ((hdr.z >> 2) & 0x30303030u)};
-        reinterpret_cast<float2*>(smem + L::dd)[(t & 3) * 128 + row] = __half22float2(*reinterpret_cast<const __half2*>(&hdr.x));
-        sp_st8(tm, h2_sub(__byte_perm(mn[0], 0x64646464u, 0x4140u), kH2Magic), h2_sub(__byte_perm(mn[0], 0x64646464u, 0x4342u), kH2Magic),
-               h2_sub(__byte_perm(mn[1], 0x64646464u, 0x4140u), kH2Magic), h2_sub(__byte_perm(mn[1], 0x64646464u, 0x4342u), kH2Magic));
+      const uint32_t mn_lo = hdr.z & 0x3F3F3F3Fu, mn_hi = ((hdr.w >> 4) & 0x0F0F0F0Fu) | ((hdr.z >> 2) & 0x30303030u);
+      // e: the power of two below the larger of 520 |d| and 63 |dmin|, so |c / e| < 4
+      const float2 dw = h2_to_f2(hdr.x);
+      const float em = fmaxf(fmaxf(520.0f * fabsf(dw.x), 63.0f * fabsf(dw.y)), 0x1p-40f);
+      const float e = __uint_as_float(__float_as_uint(em) & 0x7F800000u), re = __uint_as_float(0x7F000000u - __float_as_uint(e));
+      const float2 nd = make_float2(-dw.x * re, -dw.x * re), ndm = make_float2(-dw.y * re, -dw.y * re);
+      if (live) {
+        uint32_t ch[4], cl[4];
+        sp_offsets<0>(g_lo == 0 ? sc_lo : sc_hi, g_lo == 0 ? mn_lo : mn_hi, nd, ndm, ch[0], cl[0]);
+        sp_offsets<1>(g_lo == 0 ? sc_lo : sc_hi, g_lo == 0 ? mn_lo : mn_hi, nd, ndm, ch[1], cl[1]);
+        if (kU == 2) {
+          sp_offsets<0>(sc_hi, mn_hi, nd, ndm, ch[2], cl[2]);
+          sp_offsets<1>(sc_hi, mn_hi, nd, ndm, ch[3], cl[3]);
+        }
+        if (kU == 4) {   // this warpgroup's two groups: blocks 0 to 3 or 4 to 7
+          if (KH == 1) { sp_st2x2(tc + 2 * g_lo, ch[0], ch[1]); sp_st2x2(tc + 8 + 2 * g_lo, cl[0], cl[1]); }
+          else sp_st4x2(tc + 4 * g_lo, ch[0], ch[1], cl[0], cl[1]);
+        } else if (KH == 1) {
+          sp_st4x2(tc, ch[0], ch[1], ch[2], ch[3]);
+          sp_st4x2(tc + 8, cl[0], cl[1], cl[2], cl[3]);
+        } else {
+          sp_st4x2(tc, ch[0], ch[1], cl[0], cl[1]);
+          sp_st4x2(tc + 8, ch[2], ch[3], cl[2], cl[3]);
+        }
+        if (g_lo == 0) reinterpret_cast<float2*>(smem + L::dd)[(t & 3) * 128 + row] = make_float2(dw.x * 0x1p-8f, e * 0.0625f);
       }
       sp_wait_st();
       tc_before();
@@ -456,7 +506,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) grouped_split_q4k_kernel(const 
             if (!wait(d_full(par, buf), use & 1u)) { ok = false; break; }
             tc_after();
             const float2 dd = reinterpret_cast<const float2*>(smem + L::dd)[(t & 3) * 128 + row];
-            const float2 d2 = make_float2(dd.x, dd.x), nd2 = make_float2(-dd.y, -dd.y);
+            const float2 d2 = make_float2(dd.x, dd.x), e2 = make_float2(dd.y, dd.y);
             const uint32_t td = lane_base + buf * 96;
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
@@ -465,7 +515,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) grouped_split_q4k_kernel(const 
                 tc_ld16(td + 16 * c, p0);
                 tc_ld8(td + 64 + 8 * c, m0);
                 tc_wait_ld();
-                sp_fold8(acc + 8 * c, p0, m0, scl + kh * kNT + 8 * c, d2, nd2);
+                sp_fold8(acc + 8 * c, p0, m0, scl + kh * kNT + 8 * c, d2, e2);
               }
             }
             tc_before();
@@ -571,7 +621,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) grouped_split_q4k_kernel(const 
 #pragma unroll 1
         for (int m = 0; m < PAIR; ++m, ++t) {
           const uint32_t par = t & 1u;
-          const uint32_t ta = kSpTmemA + par * 128, tm = kSpTmemMn + par * 8;
+          const uint32_t ta = kSpTmemA + par * 128, tc = kSpTmemC + par * 16;
           if (!wait(a_full(par), (t >> 1) & 1u)) { ok = false; break; }
 #pragma unroll 1
           for (int sub = 0; sub < NH * KH; ++sub) {
@@ -582,7 +632,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) grouped_split_q4k_kernel(const 
             const int n8 = (min(32, max(0, nt - 32 * hh)) + 7) >> 3;
             if (leader) {
               const uint32_t bk = bst + hh * 8192 + kh * (2 * L::kBK), ms = sst + kh * (kNT * 32) + hh * 1024;
-              if (n8 > 0) sp_group<KH, L::kBK>(buf * 96, ta + kh * 64, tm, bk, ms, n8);
+              if (n8 > 0) sp_group<KH, L::kBK>(buf * 96, ta + kh * 64, tc + kh * 8, bk, ms, n8);
               if (sub == NH * KH - 1) {
                 tc_commit(a_empty(par));
                 if (m == PAIR - 1) tc_commit(b_empty(bs));
