@@ -355,6 +355,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) grouped_split_q4k_kernel(const 
   const uint32_t mma_end = bars + 256u;
   uint32_t* tmem_slot      = reinterpret_cast<uint32_t*>(smem + L::bar + 288);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::bar + 292);
+  RingArmed* ring_end      = reinterpret_cast<RingArmed*>(smem + L::bar + 296);   // what the weight loader armed last
 
   if (warp == kSpWarpMma) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
@@ -646,17 +647,12 @@ __global__ void __launch_bounds__(kSpThreads, 1) grouped_split_q4k_kernel(const 
         if (++bs == kB) { bs = 0; bph ^= 1u; }
       }
     }
-    if (!ok && leader) {   // let the MMAs in flight finish before the CTA gives its memory back
-      tc_commit(mma_end);
-      for (uint32_t i = 0; i < (1u << 16); ++i)
-        if (mbar_try_wait(mma_end, 0u)) break;
-    }
-    __syncwarp();
   } else if (warp == kSpWarpW) {
     // ------------------------------------------------------------------ weights
     const bool leader = sp_elect();
     int e_next = group_of(0).x, s = 0;
     uint32_t ph = 1;
+    RingArmed ring;
     for (int ui = 0; ui < my_units && ok; ++ui) {
       const int e = e_next;             // requested a unit ago
       e_next = group_of(ui + 1).x;
@@ -671,6 +667,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) grouped_split_q4k_kernel(const 
 #pragma unroll
         for (int m = 0; m < PAIR; ++m) {
           if (!wait(w_empty(s), ph)) { ok = false; break; }
+          ring.arm(s, ph ^ 1u);
           if (leader) {
             const CUtensorMap* mp = MODE == 1 && m == 1 ? m1 : m0;
             const int r0 = (MODE == 1 ? ru : ru * PAIR + m) * p.tile_rows;
@@ -684,12 +681,7 @@ __global__ void __launch_bounds__(kSpThreads, 1) grouped_split_q4k_kernel(const 
         }
       }
     }
-    if (!ok || *abort_flag) {
-      // copies may still be in flight: give them time to land before the CTA's shared memory is handed on
-      for (int s = 0; s < kW; ++s)
-        for (uint32_t i = 0; i < (1u << 14); ++i)
-          if (mbar_try_wait(w_full(s), 0u) || mbar_try_wait(w_full(s), 1u)) break;
-    }
+    if (lane == 0) *ring_end = ring;
   } else if (warp == kSpWarpX) {
     // ------------------------------------------------------------------ activation rows
     unsigned long long* rowp = reinterpret_cast<unsigned long long*>(smem + L::rowp);
@@ -759,6 +751,16 @@ __global__ void __launch_bounds__(kSpThreads, 1) grouped_split_q4k_kernel(const 
   if (MODE == 0) peer_out_finish(p.po, gridDim.x);
   tc_before();
   __syncthreads();
+  if (*abort_flag) {
+    // some role gave up: the copies and MMAs still in flight end (bounded) before the CTA gives its memory back
+    if (warp == kSpWarpW && lane == 0)
+      ring_drain(*ring_end, kW, 1u << 14, [&](int s, uint32_t parity) { return mbar_try_wait(w_full(s), parity); });
+    if (warp == kSpWarpMma && sp_elect()) {
+      tc_commit(mma_end);
+      mbar_wait_bounded(mma_end, 0u, 1u << 16);
+    }
+    __syncthreads();
+  }
   if (warp == kSpWarpMma)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(*tmem_slot), "r"(512u) : "memory");
 }

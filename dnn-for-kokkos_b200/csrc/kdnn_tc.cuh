@@ -35,6 +35,7 @@
 #include <atomic>
 
 #include "kdnn_mma.cuh"
+#include "kdnn_ring.cuh"
 
 namespace kdnn {
 
@@ -259,6 +260,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) grouped_tc_q4k_kernel(const __g
   auto s_free   = [&](int b) { return bars + 208u + 8u * b; };
   uint32_t* tmem_slot      = reinterpret_cast<uint32_t*>(smem + L::bar + 224);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::bar + 228);
+  const uint32_t mma_end   = bars + 232u;   // MMAs in flight when the CTA gave up
+  RingArmed* ring_end      = reinterpret_cast<RingArmed*>(smem + L::bar + 240);   // what the producer armed last
 
   if (warp == kTcWarpMma) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
@@ -283,6 +286,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) grouped_tc_q4k_kernel(const __g
     mbar_init(red_empty, 8);
     mbar_init(ex_full, 4);
     mbar_init(ex_empty, 4);
+    mbar_init(mma_end, 1);
     *abort_flag = 0;
     fence_barrier_init();
     fence_proxy_async();
@@ -316,6 +320,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) grouped_tc_q4k_kernel(const __g
     // ------------------------------------------------------------------ producer (one thread)
     if (lane == 0) {
       uint32_t seq = 0;
+      RingArmed ring;
       int e_next = blockIdx.x < total_tiles ? ld_dep(p.groups + blockIdx.x / p.row_tiles).x : 0;
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         const int g = t / p.row_tiles, rb = t - g * p.row_tiles;
@@ -336,6 +341,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) grouped_tc_q4k_kernel(const __g
           const uint32_t bar = w_full(s);
           const uint32_t wdst = base + L::w + s * kTcWStage;
           mbar_expect_tx(bar, static_cast<uint32_t>(nbox) * (kTcBoxRows * 144));
+          ring.arm(s, use & 1u);
           if (MODE == 1) {
             tma_load_2d(wdst, m0, ks * 144, r0, bar);
             tma_load_2d(wdst + 4608, m0, ks * 144, r0 + 32, bar);
@@ -346,13 +352,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) grouped_tc_q4k_kernel(const __g
           }
         }
       }
-      if (!ok || *abort_flag) {
-        // copies of the last stages may still be in flight: give them time to land before the CTA's
-        // shared memory is handed to somebody else (bounded, the result of the launch is void anyway)
-        for (int s = 0; s < kStages; ++s)
-          for (uint32_t i = 0; i < (1u << 16); ++i)
-            if (mbar_try_wait(w_full(s), 0u) || mbar_try_wait(w_full(s), 1u)) break;
-      }
+      *ring_end = ring;
     }
   } else if (warp >= kTcUnpackWarp0 && warp < kTcUnpackWarp0 + 8) {
     // ------------------------------------------------------------------ unpack
@@ -659,6 +659,17 @@ __global__ void __launch_bounds__(kTcThreads, 1) grouped_tc_q4k_kernel(const __g
   if (MODE == 0) peer_out_finish(p.po, gridDim.x);
   tc_before();
   __syncthreads();
+  if (*abort_flag) {
+    // some role gave up: the copies and MMAs still in flight end (bounded, the result of the launch is void anyway) before
+    // the CTA's shared memory and tensor memory are handed to somebody else
+    if (warp == kTcWarpProducer && lane == 0)
+      ring_drain(*ring_end, kStages, 1u << 14, [&](int s, uint32_t parity) { return mbar_try_wait(w_full(s), parity); });
+    if (warp == kTcWarpMma && lane == 0) {
+      tc_commit(mma_end);
+      mbar_wait_bounded(mma_end, 0u, 1u << 16);
+    }
+    __syncthreads();
+  }
   if (warp == kTcWarpMma)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTcCols) : "memory");
 }
