@@ -6,8 +6,9 @@
 //
 // Numerics. Inside a 256-element super-block the weight is d * (sc * q) - dmin * mn, 6-bit sc and 4-bit q. The tensor core
 // accumulates in fp32 and TRUNCATES, so what it sums has to be exact or small beside the result:
-//   * A = sc * q - t is an integer that fp16 holds exactly (t = 8 sc, or the nearest number to it that lets one fp16 fma
-//     form A): weights around zero, so that activations of one sign do not build a large sum that the min term takes off again;
+//   * A = sc * q - t is an integer that fp16 holds exactly, t about 7 sc in the even and 8 sc in the odd sub-blocks (what one
+//     fp16 fma can form): weights around zero, so that activations of one sign build no large sum that the min term takes
+//     off again, and what is left of it (c below) has both signs;
 //   * the rest of the weight is one number per 32 elements, c = d * t - dmin * mn, formed in fp32 and multiplied with the
 //     block's activation sum in a product of its own: c relative to a power of two e as two fp16 parts, the sum as two;
 //   * the activation row is written once (split_store_lane8) as two fp16 parts of  v = q * (256 * d / D),  D the largest d
@@ -93,8 +94,8 @@ __device__ __forceinline__ void split_store_lane8(uint8_t* row, size_t K, int b,
     n2 += __shfl_xor_sync(0xffffffffu, n2, o);                        // |v|^2 of the group
     if (o >= 4) s1 += __shfl_xor_sync(0xffffffffu, s1, o);            // its blocks' |sum|
   }
-  // u: the power of two at or above max(600 |v|, 96 sum of |block sums of v|) / 2^24, from 2 to 32
-  const float need = fminf(fmaxf(fmaxf(600.0f * sqrtf(n2), 1536.0f * s1) * 0x1p-24f, 2.0f), 32.0f);
+  // u: the power of two at or above max(600 |v|, 48 sum of |block sums of v|) / 2^24, from 2 to 32
+  const float need = fminf(fmaxf(fmaxf(600.0f * sqrtf(n2), 768.0f * s1) * 0x1p-24f, 2.0f), 32.0f);
   const float u = __uint_as_float((__float_as_uint(need) + 0x7FFFFFu) & 0x7F800000u);
   // this block's own step: its largest |v|, 127 * r, is 1016 to 2032 of them (2^-24 is fp16's last bit)
   const float own = fmaxf(__uint_as_float(__float_as_uint(r) & 0x7F800000u) * 0.125f, 0x1p-24f);
@@ -259,11 +260,11 @@ __device__ __forceinline__ uint32_t h2_sub(uint32_t a, uint32_t b) {
 }
 constexpr uint32_t kH2Magic = 0x64006400u;   // {1024, 1024}: the low four mantissa bits count units, the next four sixteens
 // 64 elements (32 bytes: low nibbles = one sub-block, high nibbles = the next) -> 32 words of pairs sc * q - t, each in one
-// exact fp16 fma: (1024 + q) * sc - fp16(1032 sc), an integer of at most 520, and (1024 + 16 q) * (sc / 16) - 72 sc.
+// exact fp16 fma: (1024 + q) * sc - fp16(1031 sc), an integer of at most 520, and (1024 + 16 q) * (sc / 16) - 72 sc.
 __device__ __forceinline__ void sp_unpack64(const uint4& a, const uint4& b, uint32_t sc_pair4, int j, uint32_t (&o)[32]) {
   const uint32_t s0 = h2_sub(__byte_perm(sc_pair4, 0x64646464u, 0x4040u + 0x0101u * j), kH2Magic);
   const uint32_t s1 = h2_sub(__byte_perm(sc_pair4, 0x64646464u, 0x4040u + 0x0101u * (j + 1)), kH2Magic);
-  const uint32_t c0 = h2_mul(s0, 0xE408E408u);      // -1032 * sc, rounded
+  const uint32_t c0 = h2_mul(s0, 0xE407E407u);      // -1031 * sc, rounded
   const uint32_t c1 = h2_mul(s1, 0xD480D480u);      // -72 * sc'
   const uint32_t s1d = h2_mul(s1, 0x2C002C00u);     // sc' / 16
   const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
@@ -286,7 +287,7 @@ template <int J>
 __device__ __forceinline__ void sp_offsets(uint32_t sc_pair4, uint32_t mn_pair4, float2 nd, float2 ndm, uint32_t& hi, uint32_t& lo) {
   const uint32_t sc = h2_sub(__byte_perm(sc_pair4, 0x64646464u, J == 0 ? 0x4140u : 0x4342u), kH2Magic);
   const uint32_t mn = h2_sub(__byte_perm(mn_pair4, 0x64646464u, J == 0 ? 0x4140u : 0x4342u), kH2Magic);
-  const uint32_t nt = h2_fma(sc, 0x00006400u, h2_mul(sc, 0xC800E408u));   // {1024 sc - fp16(1032 sc), -8 sc'}
+  const uint32_t nt = h2_fma(sc, 0x00006400u, h2_mul(sc, 0xC800E407u));   // {1024 sc - fp16(1031 sc), -8 sc'}
   const float2 c = ffma2(ndm, h2_to_f2(mn), fmul2(nd, h2_to_f2(nt)));
   hi = f2_to_h2(c);
   const float2 h = h2_to_f2(hi);

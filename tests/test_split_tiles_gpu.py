@@ -181,7 +181,7 @@ def _split(x, parts):
     r = np.float32(256.0) * (d / D)
     v = (q * r).astype(np.float32)
     need = np.maximum(600.0 * np.sqrt((v.astype(np.float64) ** 2).sum((2, 3), keepdims=True)),
-                      1536.0 * np.abs(q.sum(-1, keepdims=True) * r / 16.0).sum(2, keepdims=True)) / 2.0 ** 24
+                      768.0 * np.abs(q.sum(-1, keepdims=True) * r / 16.0).sum(2, keepdims=True)) / 2.0 ** 24
     u = 2.0 ** np.ceil(np.log2(np.clip(need, 2.0, 32.0)))
     step = np.minimum(u, np.maximum(2.0 ** np.floor(np.log2(np.maximum(r, 1e-30))) / 8.0, 2.0 ** -24))
     hi = (np.rint(v / step) * step).astype(np.float16)
