@@ -20,8 +20,10 @@ cudaError_t unit_dots_launch(uint32_t dt, const void* w, size_t rows, size_t col
 int gemv_take_status();
 
 size_t gemm_workspace_bytes(size_t M, size_t K);
+size_t gemm_workspace_min_bytes(size_t M, size_t K);
 cudaError_t gemm_launch(uint32_t dt, const void* w, size_t N, size_t K, const void* X, size_t ldx,
-                        size_t M, int xs, void* Y, size_t ldy, int ys, void* ws, int32_t* dots, cudaStream_t st);
+                        size_t M, int xs, void* Y, size_t ldy, int ys, void* ws, size_t ws_bytes, int32_t* dots,
+                        cudaStream_t st);
 int tile_kind();
 int set_tile_kind(int k);
 int device_sm_count();
@@ -307,14 +309,14 @@ int kdnn_b200_quant_gemm_dots(uint32_t ggml_type, const void* w, size_t N, size_
   if (M * N > static_cast<size_t>(INT_MAX)) return fail(KDNN_ERR_INVALID, "quant_gemm: M*N too large");
   if (!tile_type(ggml_type) || !kdnn::block_aligned(ggml_type, K)) return KDNN_DECLINED;
   if (!w || !X || !Y || !workspace) return KDNN_DECLINED;
-  if (workspace_bytes < kdnn::gemm_workspace_bytes(M, K)) return KDNN_DECLINED;
+  if (workspace_bytes < kdnn::gemm_workspace_min_bytes(M, K)) return KDNN_DECLINED;
   if ((reinterpret_cast<uintptr_t>(workspace) & 15u) || (reinterpret_cast<uintptr_t>(w) & 1u))
     return KDNN_DECLINED;
   if ((ggml_type == KDNN_GGML_Q4_K || ggml_type == KDNN_GGML_Q5_K) && (reinterpret_cast<uintptr_t>(w) & 15u) != 0u)
     return KDNN_DECLINED;   // 16-byte loads of the super-blocks, src/KokkosDNN_GGUFGemvInt8.hpp:741-743
   if (dots != nullptr && (ggml_type != KDNN_GGML_Q4_K || kdnn::tile_kind() < 2)) return KDNN_DECLINED;
   return cuda_result(kdnn::gemm_launch(ggml_type, w, N, K, X, ldx, M, x_scalar, Y, ldy, y_scalar,
-                                       workspace, dots, static_cast<cudaStream_t>(stream)),
+                                       workspace, workspace_bytes, dots, static_cast<cudaStream_t>(stream)),
                      "quant_gemm");
 }
 

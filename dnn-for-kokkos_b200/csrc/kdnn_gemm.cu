@@ -1,6 +1,7 @@
-// Batched GEMV / skinny GEMM Y[M,N] = X[M,K] W[N,K]^T with packed W and per-row
-// int8 activations: the grouped kernel of kdnn_grouped.cuh with one group that
-// holds all M activation rows. Row m of Y equals the decode GEMV applied to row m.
+// Batched GEMV / skinny GEMM Y[M,N] = X[M,K] W[N,K]^T with packed W and per-row int8 activations; row m of Y is the
+// decode GEMV applied to row m, up to the order of fp32 sums. Up to three rows run as GEMVs; Q4_K runs on kdnn_split.cuh (the
+// integer kernels of kdnn_tc.cuh and kdnn_mma.cuh where that does not apply), the other formats on kdnn_rowmma.cuh, and what
+// neither takes on the grouped kernel of kdnn_grouped.cuh with one group that holds all rows.
 #include "kdnn_grouped.cuh"
 #include "kdnn_mma.cuh"
 #include "kdnn_rowmma.cuh"
@@ -19,10 +20,15 @@ static size_t gemm_groups_offset(size_t M) { return 512 + ((M * sizeof(int) + 25
 static size_t gemm_items_offset(size_t M) {
   return gemm_groups_offset(M) + (((M + kTcNT - 1) / kTcNT * sizeof(int4) + 255) & ~size_t(255));
 }
-size_t gemm_workspace_bytes(size_t M, size_t K) {
-  // (rowmma_x_bytes of four rows and more is below the second figure: 10 bytes an element at four rows, 16 there)
-  const size_t a = M * (K / 64) * sizeof(ActItem), b = M * act_row_pitch_max(K);
+// What every call needs: the integer kernels' rows. A workspace of this size is served by them alone.
+size_t gemm_workspace_min_bytes(size_t M, size_t K) {
+  const size_t a = M * (K / 64) * sizeof(ActItem), b = M * act_row_pitch(K);
   return gemm_items_offset(M) + (a > b ? a : b);
+}
+// What the faster kernels need as well: split rows (4.14 bytes an element; rowmma_x_bytes of four rows and more is less).
+size_t gemm_workspace_bytes(size_t M, size_t K) {
+  const size_t least = gemm_workspace_min_bytes(M, K), want = gemm_items_offset(M) + M * split_row_pitch(K, 256);
+  return K % 256 == 0 && want > least ? want : least;
 }
 
 __global__ void gemm_setup_kernel(int M, uintptr_t w, int* offs, uintptr_t* wptr, int* list, int4* groups) {
@@ -51,8 +57,9 @@ static int gemm_tile_rows(size_t N, size_t groups) {
 }
 
 // Q4_K rows against M activation rows on the split-fp16 tensor-core kernel: the row quantizer and one tile launch.
+// `served` = false: no tensor map for this matrix, nothing was launched.
 static cudaError_t gemm_split(const void* w, size_t N, size_t K, const void* X, size_t ldx, size_t M, int xs, void* Y,
-                              size_t ldy, int ys, uint8_t* b, cudaStream_t st) {
+                              size_t ldy, int ys, uint8_t* b, bool& served, cudaStream_t st) {
   int* n_groups = reinterpret_cast<int*>(b) + 2;
   int4* groups  = reinterpret_cast<int4*>(b + gemm_groups_offset(M));
   uint8_t* xrows = b + gemm_items_offset(M);
@@ -69,8 +76,8 @@ static cudaError_t gemm_split(const void* w, size_t N, size_t K, const void* X, 
   q.box_rows = q.tile_rows; q.boxes = 1;
   const size_t unit_rows = static_cast<size_t>(q.tile_rows) * (wide ? 2 : 1);
   q.row_units = (int)((N + unit_rows - 1) / unit_rows);
-  err = tc_encode_matrix(&q.one, w, N, row_bytes_of(KDNN_GGML_Q4_K, K), q.box_rows);
-  if (err != cudaSuccess) return err;
+  served = tc_encode_matrix(&q.one, w, N, row_bytes_of(KDNN_GGML_Q4_K, K), q.box_rows) == cudaSuccess;
+  if (!served) return cudaSuccess;
   err = xs == KDNN_F32
             ? launch_split_rows<float>(static_cast<const float*>(X), ldx, (int)M, (int)K, xrows, groups, n_groups, cap, st)
             : launch_split_rows<__nv_bfloat16>(static_cast<const __nv_bfloat16*>(X), ldx, (int)M, (int)K, xrows, groups, n_groups, cap, st);
@@ -101,11 +108,12 @@ static cudaError_t gemm_rowmma(uint32_t dt, const void* w, size_t N, size_t K, c
 
 // `dots` (parity probe, tcgen05 kernel only): int32 [M][N][K/32] raw sub-block dots, or nullptr.
 cudaError_t gemm_launch(uint32_t dt, const void* w, size_t N, size_t K, const void* X, size_t ldx,
-                        size_t M, int xs, void* Y, size_t ldy, int ys, void* ws, int32_t* dots, cudaStream_t st) {
+                        size_t M, int xs, void* Y, size_t ldy, int ys, void* ws, size_t ws_bytes, int32_t* dots,
+                        cudaStream_t st) {
   uint8_t* b      = static_cast<uint8_t*>(ws);
-  // Crossover measured on a 14336 x 4096 Q4_K matrix: one GEMV kernel per activation row (6.9 us each) beats
-  // the tile kernels (23 us and up) for up to three rows; above, the split-fp16 kernel is the fastest on Q4_K (23.4 / 27.9 us at
-  // 8 / 32 rows; integer tcgen05 27.4 / 42, mma.sync 30 / 37).
+  const size_t room = ws_bytes - gemm_items_offset(M);   // bytes for quantized rows
+  // Up to three rows one GEMV launch per row is the fastest (14336 x 4096 Q4_K: 6.9 us each, the tile kernels 23 us and up);
+  // above, the split-fp16 kernel on Q4_K (8 / 32 rows: 24.5 / 28.7 us; integer tcgen05 27.4 / 42, mma.sync 30 / 37).
   int kind = tile_kind();
   if (kind == 3 && dots == nullptr) {
     if (M <= 3) {
@@ -118,13 +126,16 @@ cudaError_t gemm_launch(uint32_t dt, const void* w, size_t N, size_t K, const vo
       }
       return cudaSuccess;
     }
-    if (dt == KDNN_GGML_Q4_K && (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && tc_encode_fn() != nullptr)
-      return gemm_split(w, N, K, X, ldx, M, xs, Y, ldy, ys, b, st);
+    if (dt == KDNN_GGML_Q4_K && (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && M * split_row_pitch(K, 256) <= room) {
+      bool served = false;
+      const cudaError_t e = gemm_split(w, N, K, X, ldx, M, xs, Y, ldy, ys, b, served, st);
+      if (e != cudaSuccess || served) return e;
+    }
     // Every other format whose rows are whole 256-element groups (Q8_0 rows may not be) and start the matrix on 16 bytes
     // (its 16-byte copies step back to that boundary): 4096 x 14336 Q6_K, 16 rows 32.3 us, 433 on the dp4a kernel below.
-    if (dt != KDNN_GGML_Q4_K && K % 256 == 0 && (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && rowmma_x_bytes(M, K) <= M * act_row_pitch_max(K))
+    if (dt != KDNN_GGML_Q4_K && K % 256 == 0 && (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && rowmma_x_bytes(M, K) <= room)
       return gemm_rowmma(dt, w, N, K, X, ldx, M, xs, Y, ldy, ys, b + gemm_items_offset(M), st);
-    kind = 1;
+    kind = M <= 8 ? 2 : 1;   // the integer kernels' crossover: 27 against 30 us at 8 rows, 28 against 31 at 16
   } else if (kind == 3) {
     kind = 2;
   }

@@ -602,9 +602,12 @@ static MoeWs moe_ws_layout(size_t T, size_t S, size_t H, size_t F, size_t n_expe
   w.pos  = o; o += up(T * S * sizeof(int));
   w.groups = o; o += up((n_experts + T * S / kTcNT + 1) * sizeof(int4));
   w.ngroups = o; o += 256;
-  w.xq   = o; o += up(T * max_sz((H / 64) * sizeof(ActItem), act_row_pitch_max(H)));
+  // The split kernel has no use for the float activations, and its token rows are read before the first down row is
+  // written: its activation rows start at `act` and run into `actq`, its token rows at `xq` and run into `out`
+  // (1520 and 1496 bytes for 256 elements, of which 1096 and 1060 and rounding are taken).
   w.act  = o; o += up(T * S * F * sizeof(float));
-  w.actq = o; o += up(T * S * max_sz((F / 64) * sizeof(ActItem), act_row_pitch_max(F)));
+  w.actq = o; o += up(T * S * max_sz((F / 64) * sizeof(ActItem), act_row_pitch(F)));
+  w.xq   = o; o += up(T * max_sz((H / 64) * sizeof(ActItem), act_row_pitch(H)));
   w.out  = o; o += up(T * S * H * sizeof(float));
   w.total = o;
   return w;
@@ -926,7 +929,7 @@ cudaError_t moe_ffn_launch(const void* X, size_t ldx, size_t T, int xs,
     if (err != cudaSuccess) return err;
     if (split && e_count > 0) {
       err = moe_tiles_split(gate, up, down, n_slots, S, xs, e_count, cap, pp.groups, pp.n_groups, list, pp.xrows,
-                            b + L.actq, out, nullptr, st);
+                            b + L.act, out, nullptr, st);
       if (err != cudaSuccess) return err;
     } else if (e_count > 0) {
       err = moe_tiles_q4k(kind, gate, up, down, T, S, xs, e_first, e_count, b, L, st);
@@ -1050,10 +1053,10 @@ static ExLayout ex_layout(size_t Tl, size_t world, size_t S, size_t H) {
   const size_t T = Tl * world;
   ExLayout L{};
   size_t o = 0;
-  L.xrows = o; o += up(T * (world > 1 ? act_row_pitch(H) : act_row_pitch_max(H)));   // what travels is int8 rows
   L.idx   = o; o += up(T * S * sizeof(int32_t));
   L.rel   = o; o += up(T * S * sizeof(int32_t));
   L.wts   = o; o += up(T * S * sizeof(float));
+  L.xrows = o; o += up(T * act_row_pitch(H));   // one rank: split rows run into `out`, whose first row is written after they are read
   L.out   = o; o += up(T * S * H * sizeof(float));
   L.cnt   = o; o += up(kMaxLocalExperts * sizeof(int));
   L.xflag = o; o += 256;
@@ -1654,7 +1657,7 @@ static BlockWs block_ws_layout(size_t T, size_t S, size_t H, size_t F, size_t n_
   w.groups = o; o += up((n_experts + T * S / kTcNT + 1) * sizeof(int4));
   w.ngroups = o; o += 256;
   w.act  = o; o += up(T * S * F * sizeof(float));
-  w.actq = o; o += up(T * S * act_row_pitch_max(F));
+  w.actq = o; o += up(T * S * act_row_pitch(F));   // directly behind `act`: the split kernel's rows take both
   w.sync = o; o += 256;          // gate ticket, down ticket, epoch
   w.region = o; o += region_bytes;
   w.total = o;
@@ -1733,7 +1736,7 @@ cudaError_t moe_block_launch(const BlockArgs& a, cudaStream_t st) {
   po.epoch = reinterpret_cast<const uint32_t*>(sync + 2);
   if (split && a.e_count > 0) {
     err = moe_tiles_split(a.gate, a.up, a.down, T * S, S, a.scalar, a.e_count, cap, g.groups, g.n_groups, g.list,
-                          mine + XL.xrows, b + L.actq, by_position ? reinterpret_cast<float*>(mine + XL.out) : nullptr, &po, st);
+                          mine + XL.xrows, b + L.act, by_position ? reinterpret_cast<float*>(mine + XL.out) : nullptr, &po, st);
     if (err != cudaSuccess) return err;
   } else if (a.e_count > 0) {
     const int want = tile_kind() == 3 ? 1 : tile_kind();

@@ -63,11 +63,6 @@ constexpr int kSpExPitch = 132;                       // floats per activation r
 __host__ __device__ inline size_t split_sums_offset(size_t K) { return K * 4; }
 __host__ __device__ inline size_t split_scale_offset(size_t K, int G) { return K * 4 + K / G * 32; }
 inline size_t split_row_pitch(size_t K, int G) { return (split_scale_offset(K, G) + K / G * 4 + 255) & ~size_t(255); }
-inline size_t act_row_pitch_max(size_t K) {   // room for a row in either form
-  const size_t a = act_row_pitch(K), b = split_row_pitch(K, 128);
-  return a > b ? a : b;
-}
-inline bool split_rows_ok(size_t K) { return K % 256 == 0; }
 
 __device__ __forceinline__ uint32_t pack_half2(__half a, __half b) {
   return static_cast<uint32_t>(__half_as_ushort(a)) | (static_cast<uint32_t>(__half_as_ushort(b)) << 16);

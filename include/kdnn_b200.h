@@ -183,7 +183,8 @@ int kdnn_b200_unit_dots(uint32_t ggml_type, const void* w, size_t rows, size_t c
 
 /* ---- batched GEMV / skinny GEMM ------------------------------------------ */
 
-/* Workspace bytes for kdnn_b200_quant_gemm with M activation rows of K elements. */
+/* Workspace bytes for kdnn_b200_quant_gemm with M activation rows of K elements. A smaller workspace is accepted down to
+ * what the integer kernels need (1.94 bytes an element of X), which then serve the call. */
 size_t kdnn_b200_gemm_workspace_bytes(size_t M, size_t K);
 
 /* Y[M, N] = X[M, K] . W[N, K]^T with packed W, every activation row quantized per

@@ -120,6 +120,32 @@ def test_exchange_region_of_several_ranks_holds_int8_rows(kd, H):
         assert kd.MoeExchange.region_bytes(Tl, world, S, H) == want
 
 
+@pytest.mark.parametrize("T,S,H,F,E", [(1, 1, 256, 256, 1), (7, 1, 2048, 256, 5), (256, 8, 2048, 768, 128), (13, 2, 4096, 14336, 8)])
+def test_workspace_sizes_leave_no_room_for_one_form_twice(kd, T, S, H, F, E):
+    """The MoE workspaces are what the integer kernels need (a caller may have kept the size): the split rows lie over
+    areas that are idle at that moment. They fit: 1024 + int8 row behind SwiGLU, int8 row + S floats for the tokens."""
+    split = lambda K, G: _up(4 * K + K // G * 36)
+    items = lambda K: max(K // 64 * 96, _int8_row(K))
+    head = _up((E + 1) * 4) + 2 * _up(T * S * 4) + _up((E + T * S // 32 + 1) * 16) + 256
+    ffn = head + _up(T * items(H)) + _up(T * S * F * 4) + _up(T * S * items(F)) + _up(T * S * H * 4)
+    assert kd.moe_ffn_workspace_bytes(T, S, H, F, E) == ffn
+    region = kd.MoeExchange.region_bytes(T, 1, S, H)
+    assert region == _up(T * _int8_row(H)) + 3 * _up(T * S * 4) + _up(T * S * H * 4) + _up(4096 * 4) + 512
+    block = head + _up(T * S * F * 4) + _up(T * S * _int8_row(F)) + 256
+    assert kd.moe_block_workspace_bytes(T, 1, S, H, F, E, False) == block
+    assert kd.moe_block_workspace_bytes(T, 1, S, H, F, E, True) == block + region
+    assert T * S * split(F, 128) <= _up(T * S * F * 4) + T * S * _int8_row(F)
+    assert T * split(H, 256) <= _up(T * _int8_row(H)) + T * S * H * 4
+
+
+def test_gemm_workspace_declines_below_the_integer_kernels_need(kd):
+    M, K, N = 8, 512, 4
+    least = 512 + _up(M * 4) + _up((M + 31) // 32 * 16) + M * max(K // 64 * 96, _int8_row(K))
+    assert kd.quant_gemm_workspace_bytes(M, K) > least
+    f = kd.lib.kdnn_b200_quant_gemm
+    assert f(kd.Q4_K, 0x10000, N, K, 0x20000, K, M, 0, 0x30000, N, 0, 0x40000, least - 1, None) == kd.KDNN_DECLINED
+
+
 def test_encoders_round_trip(kd, port):
     import numpy as np
     from oracle import oracle as O

@@ -91,6 +91,33 @@ def test_moe_groups(kd, port, T, E, S, x_dtype):
     assert np.abs(Y.cpu().numpy() - ref).max() <= 1e-3 * np.abs(ref).max()
 
 
+def _least_workspace(M, K):
+    up = lambda v: (v + 255) // 256 * 256
+    row = up(K + 24 * (K // 32) + 48 * ((K // 32 + 7) // 8))
+    return 512 + up(M * 4) + up((M + 31) // 32 * 16) + M * max(K // 64 * 96, row)
+
+
+@gpu
+@pytest.mark.parametrize("fmt,M,kind", [(O.Q4_K, 5, 2), (O.Q4_K, 8, 2), (O.Q4_K, 9, 1), (O.Q4_K, 70, 1), (O.Q6_K, 4, 0), (O.Q6_K, 9, 0)])
+def test_a_workspace_of_the_integer_kernels_size_is_served_by_them(kd, fmt, M, kind):
+    N, K = 130, 768
+    w = kd.QuantWeight.from_numpy(kd.ggml_pack.random_payload(fmt, N, K, M, scale_bits=0x1C00), fmt, N, K, DEV)
+    X = torch.randn(M, K, generator=torch.Generator().manual_seed(M)).to(DEV)
+    out = []
+    for tile, nbytes in ((kd.TILE_AUTO, _least_workspace(M, K)), (kind, kd.quant_gemm_workspace_bytes(M, K))):
+        prev = kd.tile_kind(tile)
+        try:
+            Y = torch.full((M, N), float("nan"), device=DEV)
+            big = torch.full((nbytes + 256,), 7, dtype=torch.uint8, device=DEV)
+            kd.quant_gemm(X, w, Y, big[:nbytes])
+            torch.cuda.synchronize()
+            assert bool((big[nbytes:] == 7).all())
+        finally:
+            kd.tile_kind(prev)
+        out.append(Y)
+    assert torch.equal(out[0], out[1])
+
+
 # ---- how exact the sums are --------------------------------------------------------------------------
 def _rows(kind, M, K, g):
     """Activation rows, and the columns whose weights are zero."""
