@@ -73,7 +73,7 @@ class MoeExchangeC(C.Structure):
 
 
 KERNEL_AUTO, KERNEL_XREG, KERNEL_SMEM_WINDOW, KERNEL_ITEM_STREAM, KERNEL_PLAIN_LOADS = 0, 1, 2, 3, 4
-TILE_DP4A, TILE_MMA_SYNC, TILE_TCGEN05, TILE_AUTO = 0, 1, 2, 3
+TILE_DP4A, TILE_MMA_SYNC, TILE_TCGEN05, TILE_AUTO, TILE_SPLIT = 0, 1, 2, 3, 4
 
 
 def _load() -> C.CDLL:
@@ -262,7 +262,7 @@ def quant_gemv_int8_supported(dtype: int, K: int, scalar: torch.dtype = torch.fl
 
 def tile_kind(kind: int = -1) -> int:
     """Selects the kernel of the batched Q4_K calls (TILE_AUTO default = by measured crossover, TILE_TCGEN05,
-    TILE_MMA_SYNC, TILE_DP4A); returns the previous selection. A negative kind only queries."""
+    TILE_MMA_SYNC, TILE_DP4A, TILE_SPLIT); returns the previous selection. A negative kind only queries."""
     return int(lib.kdnn_b200_tile_kind(kind))
 
 

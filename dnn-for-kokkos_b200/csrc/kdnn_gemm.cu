@@ -49,7 +49,8 @@ __global__ void gemm_setup_kernel(int M, uintptr_t w, int* offs, uintptr_t* wptr
 static int gemm_tile_rows(size_t N, size_t groups) {
   const size_t sms = static_cast<size_t>(device_sm_count());
   for (size_t rounds = 1; rounds <= 64; ++rounds) {
-    const size_t per = (sms * rounds + groups - 1) / groups;   // row tiles per group for `rounds` full waves
+    const size_t per = sms * rounds / groups;   // row tiles per group for `rounds` full waves, not one CTA more
+    if (per == 0) continue;
     const size_t tr = (N + per - 1) / per;
     if (tr <= 128) return static_cast<int>(tr < 32 ? 32 : tr);
   }
@@ -89,6 +90,21 @@ static cudaError_t gemm_split(const void* w, size_t N, size_t K, const void* X, 
   return ys == KDNN_F32 ? launch_grouped_split<2, 1, 1, 1, float>(q, units, st) : launch_grouped_split<2, 1, 1, 1, __nv_bfloat16>(q, units, st);
 }
 
+// Whether the split kernel is the faster one for more than eight rows: with few super-blocks of K its fixed cost (tensor memory,
+// ring fill, the quantizer's larger rows) is not earned back, except where the mma.sync kernel needs another pass of 32 rows or
+// its 128-row CTAs leave most of the chip idle. mma.sync / split in us:
+//   K = 512    14336 x: 16 rows 10.2 / 11.6, 64 rows 15.3 / 16.1, 160 rows 25.5 / 21.2;  4096 x: 96 rows 11.0 / 11.8, 160 rows 17.3 / 15.1
+//   K = 1024   14336 x: 16 rows 13.0 / 14.7, 32 rows 15.9 / 16.0, 48 rows 18.3 / 21.2, 96 rows 30.0 / 29.3;  512 x: 16 rows 11.0 / 10.8
+//   K = 1536   14336 x: 16 rows 15.8 / 16.1, 24 rows 17.6 / 16.9;  8192 x: 9 rows 14.9 / 15.7, 48 rows 19.3 / 17.6
+//   K = 4096   14336 x: 16 rows 28.9 / 25.7, 32 rows 37.1 / 28.8, 64 rows 57 / 47
+static bool gemm_split_pays(size_t M, size_t N, size_t K) {
+  if (M <= 8) return true;
+  if (K <= 512) return M > 96;
+  if (N <= 2048) return true;
+  if (K <= 1024) return (M > 24 && M <= 32) || M > 64;
+  return K > 1536 || M > 16;
+}
+
 template <uint32_t DT>
 static cudaError_t gemm_rowmma_dt(const RmParams& p, const void* X, size_t ldx, int xs, uint8_t* xrows, cudaStream_t st) {
   return xs == KDNN_F32 ? launch_rowmma<DT, float>(p, static_cast<const float*>(X), ldx, xrows, st)
@@ -115,8 +131,8 @@ cudaError_t gemm_launch(uint32_t dt, const void* w, size_t N, size_t K, const vo
   // Up to three rows one GEMV launch per row is the fastest (14336 x 4096 Q4_K: 6.9 us each, the tile kernels 23 us and up);
   // above, the split-fp16 kernel on Q4_K (8 / 32 rows: 24.5 / 28.7 us; integer tcgen05 27.4 / 42, mma.sync 30 / 37).
   int kind = tile_kind();
-  if (kind == 3 && dots == nullptr) {
-    if (M <= 3) {
+  if (kind >= 3 && dots == nullptr) {
+    if (M <= 3 && kind == 3) {
       uint8_t* scratch = b + gemm_items_offset(M);   // room for one staged row: the workspace holds M of them
       const size_t xb = xs == KDNN_F32 ? 4 : 2, yb = ys == KDNN_F32 ? 4 : 2;
       for (size_t m = 0; m < M; ++m) {
@@ -126,7 +142,8 @@ cudaError_t gemm_launch(uint32_t dt, const void* w, size_t N, size_t K, const vo
       }
       return cudaSuccess;
     }
-    if (dt == KDNN_GGML_Q4_K && (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && M * split_row_pitch(K, 256) <= room) {
+    if (dt == KDNN_GGML_Q4_K && (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && M * split_row_pitch(K, 256) <= room &&
+        (kind == 4 || gemm_split_pays(M, N, K))) {
       bool served = false;
       const cudaError_t e = gemm_split(w, N, K, X, ldx, M, xs, Y, ldy, ys, b, served, st);
       if (e != cudaSuccess || served) return e;
@@ -136,7 +153,7 @@ cudaError_t gemm_launch(uint32_t dt, const void* w, size_t N, size_t K, const vo
     if (dt != KDNN_GGML_Q4_K && K % 256 == 0 && (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && rowmma_x_bytes(M, K) <= room)
       return gemm_rowmma(dt, w, N, K, X, ldx, M, xs, Y, ldy, ys, b + gemm_items_offset(M), st);
     kind = M <= 8 ? 2 : 1;   // the integer kernels' crossover: 27 against 30 us at 8 rows, 28 against 31 at 16
-  } else if (kind == 3) {
+  } else if (kind >= 3) {
     kind = 2;
   }
   int* offs       = reinterpret_cast<int*>(b);

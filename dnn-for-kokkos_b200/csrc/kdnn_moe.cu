@@ -19,6 +19,7 @@
 #include "kdnn_tc.cuh"
 
 #include <limits.h>
+#include <math.h>
 #include <stdlib.h>
 #include <string.h>
 
@@ -86,13 +87,12 @@ cudaError_t tc_encode_matrix_host(void* out128, const void* w, size_t rows, size
   return e;
 }
 
-// Which Q4_K tile kernel the batched calls use: 3 = by measured crossover (default: the GEMV kernel per row
-// up to 3 activation rows, the tcgen05 kernel up to 8, the mma.sync kernel beyond and for the MoE
-// feed-forward), 2 = tcgen05 + TMEM everywhere it applies, 1 = mma.sync, 0 = the CUDA-core dp4a kernel
-// (which also serves every other format). Process-wide, read per call.
+// Which tile kernel the batched Q4_K calls use (kdnn_b200_tile_kind): 3 = by measured crossover (default: gemm_launch,
+// split_pays, token_pays), 4 = the split-fp16 tcgen05 kernel wherever it applies, 2 = the integer tcgen05 kernel, 1 = mma.sync,
+// 0 = the CUDA-core dp4a kernel. Process-wide, read per call.
 static std::atomic<int> g_tile_kind{3};
 int tile_kind() { return g_tile_kind.load(std::memory_order_relaxed); }
-int set_tile_kind(int k) { return k >= 0 && k <= 3 ? g_tile_kind.exchange(k) : g_tile_kind.load(); }
+int set_tile_kind(int k) { return k >= 0 && k <= 4 ? g_tile_kind.exchange(k) : g_tile_kind.load(); }
 
 // ---- router ----------------------------------------------------------------------
 // One warp per token; the E scores live in shared memory (src/KokkosDNN_MoE.hpp:
@@ -717,12 +717,25 @@ static bool tc_covers(const kdnn_b200_weight_table* gate, const kdnn_b200_weight
   const size_t H = gate->cols, F = gate->rows;
   return gate->tma != nullptr && up->tma != nullptr && down->tma != nullptr && F % 64 == 0 && H >= 512 && F >= 256;
 }
-// Whether the split-fp16 kernel runs this call: the default selection, with the tables' descriptors at hand. (A single
-// token leaves both tile kernels mostly idle: the token kernels take it, mma.sync where its slots do not fit them.)
+// Whether the split-fp16 kernel can run this call: one of its kinds, with the tables' descriptors at hand.
 static bool split_covers(const kdnn_b200_weight_table* gate, const kdnn_b200_weight_table* up,
                          const kdnn_b200_weight_table* down) {
-  return tile_kind() == 3 && gate->tma != nullptr && up->tma != nullptr && down->tma != nullptr && gate->cols % 256 == 0 &&
+  return tile_kind() >= 3 && gate->tma != nullptr && up->tma != nullptr && down->tma != nullptr && gate->cols % 256 == 0 &&
          gate->rows % 256 == 0;
+}
+// Whether it is the faster one. A CTA owns an SM and walks whole units (128 rows of gate and up, 256 of down) super-block by
+// super-block: it needs several units per SM, or long runs, to beat the smaller and more numerous CTAs of the mma.sync
+// kernel. Units are counted over the experts that some token is likely to choose. Feed-forward, mma.sync / split in us:
+//   2048 x 768, 128 experts, top-8      1792 units, 4 rows an expert: 188 / 166   16 rows: 243 / 198   (714 units, 8 tokens: 98 / 96)
+//   4096 x 14336, 8 experts, top-2      1024 units, 8 rows: 363 / 332   448 units, 2 tokens: 165 / 224
+//   2048 x 1536, 60 experts, top-4      1200 units, 2 rows: 146 / 137   500 units, 8 tokens: 85 / 92
+//   4096 x 1536, 16 experts, top-2       448 units, 8 rows: 110 / 109   4 rows: 99 / 107
+//   1024 x 512, 32 experts, top-4        256 units, 32 rows: 55 / 63    50 rows: 67 / 56   97 rows: 104 / 86
+static bool split_pays(size_t T, size_t S, size_t n_experts, size_t e_count, size_t H, size_t F) {
+  if (tile_kind() == 4) return true;
+  const double rows = static_cast<double>(T * S) / static_cast<double>(n_experts);   // an expert's mean run
+  const double units = -static_cast<double>(e_count) * expm1(-rows) * static_cast<double>(F / 128 + H / 256);
+  return units >= 900.0 || (rows >= 8.0 && units >= 400.0) || rows >= 48.0;
 }
 // Activation rows per group: 64 once the experts' mean run is longer than 32 (weights are then unpacked half as often).
 static int split_cap(size_t n_slots, size_t n_experts) { return n_slots > 32 * n_experts ? 64 : 32; }
@@ -851,6 +864,15 @@ constexpr size_t kTokenSmem = 48 * 1024;   // quantized rows of one CTA: what a 
 static bool token_covers(size_t S, size_t H, size_t F) {
   return H / 64 * sizeof(ActItem) <= kTokenSmem && S * (F / 64) * sizeof(ActItem) <= kTokenSmem && S <= 65535;
 }
+// Whether they are the faster ones: each of the H / 8 CTAs of the down kernel quantizes all S * F activations, so many
+// slots of long rows over few output rows go through the tiles. Q4_K, tiles / token kernels in us: 1024 x 1024 top-8 33 / 29,
+// x 2048 top-8 38 / 45, x 3584 top-4 41 / 37, top-8 55 / 75; 2048 x 2048 top-8 46 / 49, x 5120 top-4 66 / 56; 3072 x 3072
+// top-8 87 / 77; 4096 x 4096 top-8 118 / 93. Against the dp4a tiles of the other formats (Q6_K down): 1536 x 3072 top-8
+// 142 / 127, 1024 x 3584 top-8 108 / 126.
+static bool token_pays(size_t S, size_t H, size_t F, bool q4k) {
+  if (!q4k) return S <= 6 || S * F <= 16 * H;
+  return S <= 4 || S * F <= 14336 || (H >= 3072 && S * F <= 8 * H);
+}
 
 template <uint32_t DT>
 static cudaError_t token_gate_up(const TokenParams& p, int xs, cudaStream_t st) {
@@ -905,12 +927,12 @@ cudaError_t moe_ffn_launch(const void* X, size_t ldx, size_t T, int xs,
   ActItem* xq   = reinterpret_cast<ActItem*>(b + L.xq);
   ActItem* actq = reinterpret_cast<ActItem*>(b + L.actq);
   float* out = reinterpret_cast<float*>(b + L.out);
-  if (T == 1 && tile_kind() == 3 && token_covers(S, H, F))
+  const bool q4k = gate->ggml_type == KDNN_GGML_Q4_K && down->ggml_type == KDNN_GGML_Q4_K;
+  if (T == 1 && tile_kind() == 3 && token_covers(S, H, F) && token_pays(S, H, F, q4k))
     return moe_token_launch(X, xs, gate, up, down, idx, wts, S, Y, ys, e_first, e_count, act, st);
   const int n_slots = static_cast<int>(T * S);
-  const bool all_q4k = gate->ggml_type == KDNN_GGML_Q4_K && down->ggml_type == KDNN_GGML_Q4_K &&
-                       (reinterpret_cast<uintptr_t>(ws) & 15u) == 0;
-  const int want = tile_kind() == 3 ? 1 : tile_kind();   // measured: the mma.sync kernel is the faster one here
+  const bool all_q4k = q4k && (reinterpret_cast<uintptr_t>(ws) & 15u) == 0;
+  const int want = tile_kind() >= 3 ? 1 : tile_kind();   // where the split kernel does not run: mma.sync is the faster integer kernel
   const int kind = !all_q4k ? 0 : (want == 2 && !tc_covers(gate, up, down)) ? 1 : want;
   cudaError_t err;
   if (kind != 0 && moe_sort_smem(e_count, T) <= kPrepSmemLimit) {
@@ -921,7 +943,7 @@ cudaError_t moe_ffn_launch(const void* X, size_t ldx, size_t T, int xs,
     pp.offs = offs; pp.list = list; pp.pos = pos;
     pp.groups = reinterpret_cast<int4*>(b + L.groups); pp.n_groups = reinterpret_cast<int*>(b + L.ngroups);
     pp.X = e_count > 0 ? X : nullptr; pp.ldx = ldx; pp.T = (int)T; pp.H = (int)H;
-    const bool split = T > 1 && split_covers(gate, up, down);
+    const bool split = T > 1 && split_covers(gate, up, down) && split_pays(T, S, gate->n_experts, e_count, H, F);
     const int cap = split ? split_cap(n_slots, gate->n_experts) : kTcNT;
     pp.cap_log2 = cap == 64 ? 6 : 5;
     pp.xrows = b + L.xq; pp.x_pitch = split ? split_row_pitch(H, 256) : act_row_pitch(H);
@@ -1691,7 +1713,7 @@ cudaError_t moe_block_launch(const BlockArgs& a, cudaStream_t st) {
   for (size_t r = 0; r < world; ++r) g.region[r] = regions[r];
   // Rows that travel are int8 rows whatever this rank's tables and tile kind are: a peer reads them in ITS form, and all
   // integer kernels share that one (3968 bytes a row at hidden 2048, the split form 8480).
-  const bool split = a.world == 1 && split_covers(a.gate, a.up, a.down);
+  const bool split = a.world == 1 && T > 1 && split_covers(a.gate, a.up, a.down) && split_pays(T, S, E, a.e_count, H, F);
   const int cap = split ? split_cap(T * S, E) : kTcNT;
   g.split = split; g.cap_log2 = cap == 64 ? 6 : 5;
   g.L = XL; g.x_pitch = split ? split_row_pitch(H, 256) : act_row_pitch(H);
@@ -1739,7 +1761,7 @@ cudaError_t moe_block_launch(const BlockArgs& a, cudaStream_t st) {
                           mine + XL.xrows, b + L.act, by_position ? reinterpret_cast<float*>(mine + XL.out) : nullptr, &po, st);
     if (err != cudaSuccess) return err;
   } else if (a.e_count > 0) {
-    const int want = tile_kind() == 3 ? 1 : tile_kind();
+    const int want = tile_kind() >= 3 ? 1 : tile_kind();
     const int kind = (want == 2 && !tc_covers(a.gate, a.up, a.down)) || want == 0 ? 1 : want;
     const int n_slots = (int)(T * S);
     int* offs = reinterpret_cast<int*>(b + L.offs);

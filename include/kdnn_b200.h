@@ -207,12 +207,19 @@ int kdnn_b200_quant_gemm_dots(uint32_t ggml_type, const void* w, size_t N, size_
                               void* workspace, size_t workspace_bytes, void* stream);
 
 /* Which kernel the batched Q4_K calls (quant_gemm, moe_ffn, moe_block) use from now on, process-wide:
- * 3 = by measured crossover (the default: quant_gemm runs the GEMV kernel per row up to 3 activation rows,
- * the tcgen05 kernel up to 8, the mma.sync kernel beyond; the MoE feed-forward runs the mma.sync kernel),
- * 2 = tcgen05.mma + TMEM fed by tensor-map TMA wherever it applies, 1 = mma.sync m16n8k32, 0 = the
- * CUDA-core dp4a kernel that serves every other format. Returns the previous kind; kind < 0 only queries.
- * A tuning knob in the sense of Int8Layout (src/KokkosDNN_GGUFGemvInt8.hpp:604-608); results agree
- * within fp32 summation order. */
+ * 3 = by measured crossover (the default). quant_gemm: the GEMV kernel per row up to 3 activation rows, above that the
+ *     split-fp16 tcgen05 kernel, or an integer kernel where that is faster (more than 8 rows, small K), where the workspace
+ *     is the smaller size or the driver has no tensor-map encoder. moe_ffn / moe_block: the split-fp16 kernel where the experts chosen give
+ *     it enough work and their tables carry TMA descriptors, the mma.sync kernel otherwise and with several ranks; moe_ffn of
+ *     ONE token: two kernels of its own, every format, unless many slots of long rows meet few output rows,
+ * 4 = the split-fp16 kernel wherever it applies, 2 = integer tcgen05.mma + TMEM fed by tensor-map TMA wherever it applies,
+ * 1 = mma.sync m16n8k32, 0 = the CUDA-core dp4a kernel.
+ * Other formats: quant_gemm of Q5_K, Q6_K and Q8_0 runs an int8 mma.sync kernel (kind 3 and 4, K a multiple of 256, a 16-byte
+ * aligned matrix, room in the workspace) or the dp4a kernel; moe_ffn of several tokens the dp4a kernel.
+ * Returns the previous kind; kind < 0 only queries. A tuning knob in the sense of Int8Layout
+ * (src/KokkosDNN_GGUFGemvInt8.hpp:604-608). The integer kinds add exact per-32 integer dots in fp32; the split kernel sums fp16
+ * products of the activations in two parts, exact to 22 bits of a 32-element block as long as the block is within 2^15 of the
+ * largest one in its 256 elements (128 behind SwiGLU). Error against float64 of either: 1e-7 to 1e-6 of the result (2-norm). */
 int kdnn_b200_tile_kind(int kind);
 
 /* ---- MoE ------------------------------------------------------------------ */
@@ -237,8 +244,8 @@ typedef struct {
   size_t rows, cols, row_bytes;
   size_t n_experts;
   const void* tma;       /* device array [n_experts] of 128-byte TMA descriptors written by
-                            kdnn_b200_weight_table_tma_encode, or NULL (the tcgen05 tile kernel then
-                            leaves the call to the mma.sync kernel) */
+                            kdnn_b200_weight_table_tma_encode, or NULL (both tcgen05 kernels, split-fp16
+                            and integer, then leave the call to the mma.sync kernel) */
 } kdnn_b200_weight_table;
 
 /* Bytes of the descriptor array of a table with n_experts entries (128 each). */

@@ -36,12 +36,20 @@ def _gemm(kd, w, X, dtype=torch.float32):
     return Y
 
 
+@pytest.fixture
+def split_kernel(kd):
+    """The kernel under test whatever the size rules of the default kind prefer."""
+    prev = kd.tile_kind(kd.TILE_SPLIT)
+    yield
+    kd.tile_kind(prev)
+
+
 # one row tile per CTA: fewer rows than a tile, one past it, odd row counts; 8-row steps of the activation rows and
 # one past each; one super-block and odd numbers of them. Last two: two row tiles and 64-row groups.
 @gpu
 @pytest.mark.parametrize("N,K,M", [(1, 256, 4), (33, 256, 8), (97, 512, 9), (128, 768, 17), (129, 1280, 25), (300, 512, 31),
                                    (257, 256, 32), (130, 768, 33), (9600, 256, 200), (19001, 768, 65)])
-def test_gemm_edges(kd, N, K, M):
+def test_gemm_edges(kd, split_kernel, N, K, M):
     w = kd.QuantWeight.from_numpy(kd.ggml_pack.random_payload(O.Q4_K, N, K, N + M, scale_bits=0x1C00), O.Q4_K, N, K, DEV)
     g = torch.Generator().manual_seed(M)
     X = torch.randn(M, K, generator=g)
@@ -55,7 +63,7 @@ def test_gemm_edges(kd, N, K, M):
 
 
 @gpu
-def test_a_non_finite_row_stays_alone(kd):
+def test_a_non_finite_row_stays_alone(kd, split_kernel):
     N, K, M = 200, 512, 12
     w = kd.QuantWeight.from_numpy(kd.ggml_pack.random_payload(O.Q4_K, N, K, 3, scale_bits=0x1C00), O.Q4_K, N, K, DEV)
     X = torch.randn(M, K, generator=torch.Generator().manual_seed(1))
@@ -69,7 +77,7 @@ def test_a_non_finite_row_stays_alone(kd):
 @gpu
 @pytest.mark.parametrize("T,E,S", [(100, 4, 2), (7, 5, 1), (65, 1, 1)])   # runs past 32 rows take 64-row groups
 @pytest.mark.parametrize("x_dtype", [torch.float32, torch.bfloat16])
-def test_moe_groups(kd, port, T, E, S, x_dtype):
+def test_moe_groups(kd, port, split_kernel, T, E, S, x_dtype):
     H, F = 512, 768                          # three super-blocks of the down projection
     mk = lambda r, c, s: [kd.ggml_pack.synth_weight(O.Q4_K, r, c, s + e, std=0.05) for e in range(E)]
     gate, up, down = mk(F, H, 1), mk(F, H, 100), mk(H, F, 200)
@@ -165,18 +173,18 @@ def test_error_by_distribution(kd, kind, one_sign_weights):
         w = kd.QuantWeight.from_numpy(kd.ggml_pack.quantize(O.Q4_K, W.astype(np.float32)), O.Q4_K, N, K, DEV)
         want, _ = _exact(kd, w, x)
         err = {}
-        for tile in (kd.TILE_AUTO, kd.TILE_MMA_SYNC):
+        for tile in (kd.TILE_SPLIT, kd.TILE_MMA_SYNC):
             prev = kd.tile_kind(tile)
             try:
                 err[tile] = _rel(_gemm(kd, w, x).cpu().numpy(), want)
             finally:
                 kd.tile_kind(prev)
-        assert err[kd.TILE_AUTO] <= min(1e-6, max(2e-7, 1.25 * err[kd.TILE_MMA_SYNC])), (N, K, M, err)
+        assert err[kd.TILE_SPLIT] <= min(1e-6, max(2e-7, 1.25 * err[kd.TILE_MMA_SYNC])), (N, K, M, err)
 
 
 @gpu
 @pytest.mark.parametrize("T", [20, 40])
-def test_down_product_of_known_activations(kd, T):
+def test_down_product_of_known_activations(kd, split_kernel, T):
     """One expert with weight 1: the down product (128-element groups) against float64 of the activations as
     quantized. A gate or up product that rounds the other way turns an activation by one int8 step in a few rows, so the
     bound is on three rows of four: 1e-6."""
