@@ -474,8 +474,8 @@ def run_ours(args):
     by_batch = {}
     copies = q4
     N_, K_ = 14336, 4096
-    paths = {1: "GEMV kernel per row", 2: "GEMV kernel per row", 4: "tcgen05 tile kernel", 8: "tcgen05 tile kernel",
-             16: "mma.sync tile kernel", 32: "mma.sync tile kernel"}
+    paths = {1: "GEMV kernel per row", 2: "GEMV kernel per row", 4: "split-fp16 tcgen05 tile kernel",
+             8: "split-fp16 tcgen05 tile kernel", 16: "split-fp16 tcgen05 tile kernel", 32: "split-fp16 tcgen05 tile kernel"}
     for M in (1, 2, 4, 8, 16, 32):
         X = torch.randn(M, K_, generator=torch.Generator().manual_seed(SEED + M)).to(torch.bfloat16).to(dev)
         Y = torch.empty(M, N_, dtype=torch.float32, device=dev)
@@ -601,7 +601,7 @@ def run_ours(args):
         else:
             small = moe_bench.StackConfig(layers=8)
             per_kind = {}
-            for kind, nm in ((1, "mma.sync"), (2, "tcgen05")):
+            for kind, nm in ((3, "auto"), (1, "mma.sync"), (2, "integer tcgen05")):
                 r = moe_bench.bench_moe_stack(kd, dev, rank, world, steps=steps_m, warmup=3, peak=peak, cfg=small,
                                               tile_kind=kind)
                 per_kind[nm] = r["us_per_layer"]
@@ -609,7 +609,7 @@ def run_ours(args):
             c4cfg = moe_bench.StackConfig(layers=2, hidden=4096, ffn=14336, experts=8, top_k=2, tokens=64)
             c4 = {"config": "8 experts, top-2, hidden 4096, FFN 14336, 64 tokens, one block = 792.7 MB of packed experts",
                   "us_per_layer": {}}
-            for kind, nm in ((1, "mma.sync"), (2, "tcgen05")):
+            for kind, nm in ((3, "auto"), (1, "mma.sync"), (2, "integer tcgen05")):
                 r = moe_bench.bench_moe_stack(kd, dev, rank, world, steps=steps_m, warmup=3, peak=peak, cfg=c4cfg,
                                               tile_kind=kind)
                 c4["us_per_layer"][nm] = r["us_per_layer"]

@@ -242,7 +242,7 @@ def bench_moe_stack(kd, dev, rank: int, world: int, steps: int = 5, warmup: int 
     del graph          # its kernels name the exchange regions
     stack.close()
     layer_bytes = cfg.layer_bytes()
-    names = {3: "auto (mma.sync for the MoE tiles)", 2: "tcgen05 + TMEM", 1: "mma.sync", 0: "dp4a"}
+    names = {4: "split-fp16 tcgen05", 3: "auto (split-fp16 tcgen05 or mma.sync by size)", 2: "tcgen05 + TMEM", 1: "mma.sync", 0: "dp4a"}
     return {
         "metric": "moe_decode_tokens_per_s", "value": cfg.tokens / (ms * 1e-3), "unit": "tokens/s",
         "n_gpus": world, "ms_per_step": ms, "scaling": "strong",
