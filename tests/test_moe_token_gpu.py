@@ -50,3 +50,41 @@ def test_token_equals_general_path(kd, fmts, H, F, S, dtype):
         out.append(Y.cpu().numpy().astype(np.float64))
     assert np.isfinite(out[1]).all() and np.abs(out[1]).max() > 0
     assert np.abs(out[0] - out[1]).max() <= np.abs(out[1]).max() / 127
+
+
+def _product(kd, w, x):
+    """float64 W . q(x) with the int8-quantized row; weights from the bit-exact dequantizer."""
+    dense = torch.empty((w.rows, w.cols), dtype=torch.float32, device=DEV)
+    kd.dequant_to_dense(w, dense)
+    b = x.reshape(-1, 32).astype(np.float32)
+    amax = np.abs(b).max(-1, keepdims=True)
+    inv = np.divide(np.float32(127.0), amax, out=np.zeros_like(amax), where=amax > 0)
+    q = np.clip(np.rint(b * inv), -127, 127).astype(np.float64) * (amax / np.float32(127.0)).astype(np.float64)
+    return dense.cpu().numpy().astype(np.float64) @ q.reshape(-1)
+
+
+@pytest.mark.parametrize("fmts", [(O.Q4_K, O.Q4_K), (O.Q4_K, O.Q6_K), (O.Q8_0, O.Q4_K)])
+def test_token_against_float64(kd, fmts):
+    """fp32 outputs of eight tokens, one expert: relative 2-norm at most 1e-6 for the median token (fp32 sums of at most 768 and
+    512 terms; a product that rounds the other way turns an activation by one int8 step in a token here and there). The bf16
+    output is the fp32 output rounded once."""
+    H, F = 768, 512
+    mk = lambda fmt, r, c, s: kd.QuantWeight.from_numpy(kd.ggml_pack.synth_weight(fmt, r, c, s, std=0.05), fmt, r, c, DEV)
+    gate, up, down = mk(fmts[0], F, H, 1), mk(fmts[0], F, H, 2), mk(fmts[1], H, F, 3)
+    tabs = [kd.make_quant_weight_table([w]) for w in (gate, up, down)]
+    idx, wts = torch.zeros(1, 1, dtype=torch.int32, device=DEV), torch.ones(1, 1, device=DEV)
+    err = []
+    for seed in range(8):
+        x = torch.randn(1, H, generator=torch.Generator().manual_seed(seed))
+        out = {}
+        for dtype in (torch.float32, torch.bfloat16):
+            Y = torch.full((1, H), float("nan"), dtype=dtype, device=DEV)
+            ws = torch.zeros(kd.moe_ffn_workspace_bytes(1, 1, H, F, 1), dtype=torch.uint8, device=DEV)
+            kd.moe_ffn(x.to(DEV), *tabs, idx, wts, Y, ws)
+            torch.cuda.synchronize()
+            out[dtype] = Y
+        assert torch.equal(out[torch.bfloat16], out[torch.float32].to(torch.bfloat16))
+        a, b = _product(kd, gate, x.numpy()), _product(kd, up, x.numpy())
+        want = _product(kd, down, (a / (1.0 + np.exp(-a)) * b).astype(np.float32))
+        err.append(np.linalg.norm(out[torch.float32].cpu().numpy()[0] - want) / np.linalg.norm(want))
+    assert np.median(err) <= 1e-6, err
