@@ -14,8 +14,10 @@ DEV = "cuda:0"
 
 
 # fewer items than lanes, as many, one more; a row count that leaves the last CTA short (256 = 16 x 16, 768 = 96 x 8);
-# the largest quantized slots that fit 48 KB of shared memory (8 x 4096) and the first that do not (8 x 4352)
-@pytest.mark.parametrize("H,F,S", [(256, 256, 1), (2048, 768, 8), (2304, 512, 3), (512, 4096, 8), (512, 4352, 8)])
+# the largest quantized slots that fit 48 KB of shared memory (4 x 8192) and the first that do not (4 x 8448); eight
+# slots of that size, which go through the tiles
+@pytest.mark.parametrize("H,F,S", [(256, 256, 1), (2048, 768, 8), (2304, 512, 3), (512, 8192, 4), (512, 8448, 4), (512, 4096, 8),
+                                   (512, 4352, 8)])
 @pytest.mark.parametrize("fmts", [(O.Q4_K, O.Q4_K), (O.Q4_K, O.Q6_K), (O.Q5_K, O.Q8_0), (O.Q6_K, O.Q5_K)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_token_equals_general_path(kd, fmts, H, F, S, dtype):
